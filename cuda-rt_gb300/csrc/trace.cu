@@ -1,7 +1,8 @@
 // trace.cu -- traversal and the pixel kernel on sm_103a.
 //
 // k_trace<ANY>  closest hit (BVH_d::intersect) or first hit in left-first
-//               DFS order (BVH_d::intersectAny) for a batch of double rays.
+//               DFS order (BVH_d::intersectAny) for a batch of double rays,
+//               the lanes of a warp refilled as their rays end.
 // k_pixels      runRayTracerKernelRec (kernels/raytracer.cu:95-166) with
 //               traceRay (raytracer.cu:169-249), Material::shade
 //               (kernels/material.cu:6-40) and the positional Light
@@ -19,37 +20,41 @@ namespace crt {
 
 namespace {
 
+// Batched rays: a warp owns every stride-th chunk of `per` consecutive rays
+// (per <= 32: neighbouring rays share their lanes' nodes, and the chunks
+// spread the costly regions of the batch over the warps) and refills its
+// lanes from them.
 template <bool ANY>
-__global__ void __launch_bounds__(128) k_trace(DScene S, const double* __restrict__ rays, int64_t n,
+__global__ void __launch_bounds__(128) k_trace(DScene S, const double* __restrict__ rays, int64_t n, int per,
                                                int* __restrict__ ids, double* __restrict__ tout,
                                                double* __restrict__ nout) {
   float rb[6], B, D;
   scene_consts(S, rb, B, D);
-  const int lane = threadIdx.x & 31;
-  // warp-uniform loop (the traversal is warp-synchronous): lanes past n ride along
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-    const int64_t i = base + lane;
-    const bool live = i < n;
-    RayC rc;
-    if (live) {
-      const double* r = rays + 6 * i;
-      ray_setup(rc, r[0], r[1], r[2], r[3], r[4], r[5], B, D);
-    } else {
-      ray_setup(rc, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, B, D);
-    }
-    HitRec h;
-    const int res = traverse<ANY>(S, rc, rb, h, live);
-    if (res < 0) atomicOr(&S.g->err, kErrStack);
-    if (!live) continue;
-    const bool hit = res > 0;
-    ids[i] = hit ? h.id : -1;
-    if (tout) tout[i] = hit ? h.t : 0.0;
-    if (!ANY && nout && hit) {
-      const D3 N = hit_normal(S, h);
-      nout[3 * i] = N.x, nout[3 * i + 1] = N.y, nout[3 * i + 2] = N.z;
-    }
-  }
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t chunks = (n + per - 1) / per;
+  const int64_t mine = w < chunks ? (chunks - 1 - w) / warps + 1 : 0;  // chunks w, w + warps, ...
+  auto at = [&](int64_t i) { return (w + (i / per) * warps) * per + i % per; };
+  walk_queue<ANY>(
+      S, rb, (int)(mine * per),
+      [&](int i, RayC& rc) {
+        const int64_t k = at(i);
+        if (k >= n) return false;
+        const double* r = rays + 6 * k;
+        ray_setup(rc, r[0], r[1], r[2], r[3], r[4], r[5], B, D);
+        return true;
+      },
+      [&](int i, const RayC&, int res, const HitRec& h) {
+        const int64_t k = at(i);
+        if (res < 0) atomicOr(&S.g->err, kErrStack);
+        const bool hit = res > 0;
+        ids[k] = hit ? h.id : -1;
+        if (tout) tout[k] = hit ? h.t : 0.0;
+        if (!ANY && nout && hit) {
+          const D3 N = hit_normal(S, h);
+          nout[3 * k] = N.x, nout[3 * k + 1] = N.y, nout[3 * k + 2] = N.z;
+        }
+      });
 }
 
 // One scene: warps claim tiles of 32 / G pixels of rows [row0, row1).
@@ -130,12 +135,18 @@ cudaError_t launch_trace(const DScene& S, const double* rays, int64_t n, bool an
   else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_trace<false>, 128, 0);
   if (bps <= 0) bps = 1;
-  const int64_t need = (n + 127) / 128;
+  // few rays are spread over more warps: a walk's latency, not the lanes,
+  // then bounds the call (4096 rays: 248 us with 32 to a warp, 166 us with 2,
+  // both with the 100 us rebuild before them)
+  const int64_t warps = (int64_t)num_sms() * bps * 4;
+  int per = 32;
+  while (per > 2 && (n + per - 1) / per < warps) per /= 2;
+  const int64_t need = ((n + per - 1) / per + 3) / 4;
   const int grid = (int)(need < (int64_t)num_sms() * bps ? need : (int64_t)num_sms() * bps);
   if (any)
-    k_trace<true><<<grid, 128, 0, st>>>(S, rays, n, ids, t, nullptr);
+    k_trace<true><<<grid, 128, 0, st>>>(S, rays, n, per, ids, t, nullptr);
   else
-    k_trace<false><<<grid, 128, 0, st>>>(S, rays, n, ids, t, normals);
+    k_trace<false><<<grid, 128, 0, st>>>(S, rays, n, per, ids, t, normals);
   return cudaGetLastError();
 }
 

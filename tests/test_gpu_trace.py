@@ -106,3 +106,21 @@ def test_bad_input_reports_status(cuda):
     with pytest.raises(crt.CrtError) as e:
         crt.Scene(nan)
     assert e.value.status == 1
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 4865, 77_825, 156_000])
+@pytest.mark.parametrize("any_hit", [False, True])
+def test_trace_ray_counts(cuda, n, any_hit):
+    """Batches that fill part of a warp's lanes, that spread two rays to a warp, and that refill the lanes
+    (more rays than resident lanes): every ray bit for bit as the oracle's."""
+    import crt
+    from crt import data
+    from oracle.oracle import OracleScene
+    m = data.soup(3000, seed=4, sigma=0.05)
+    g, o = crt.Scene(m), OracleScene(m)
+    rays = _random_rays(np.random.default_rng(n), n, np.array([0, 0, -3.0]), 1.5)
+    gi, gt = g.trace(rays, any_hit=any_hit)
+    oi, ot, _ = o.trace(rays, any_hit=any_hit)
+    assert_equal(gi, oi, "ids")
+    assert_equal(gt, ot, "t")
+    g.check()
