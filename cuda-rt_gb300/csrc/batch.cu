@@ -273,9 +273,10 @@ crt_status crt_batch_create(const crt_mesh_desc* meshes, const crt_batch_view* v
   const size_t sz[] = {12 * (size_t)V, 12 * (size_t)Nn, 12 * (size_t)N, 12 * (size_t)N, 4 * (size_t)N,
                        sizeof(DMat) * (size_t)Mat, 4 * (size_t)N, 4 * (size_t)(M + 1), 4 * (size_t)kLaneOptions * (M + 1),
                        5 * 4 * (size_t)N, 4 * 4 * (size_t)kRadix, 4 * 4 * (size_t)tiles * kRadix,
-                       4 * (size_t)(NI + N), 4 * (size_t)(NI > 0 ? NI : 1), 0,
+                       4 * (size_t)(NI + N), 4 * (size_t)(NI > 0 ? NI : 1), 32 * (size_t)(NI > 0 ? NI : 1),
                        sizeof(LeafTri) * (size_t)N, sizeof(SceneGlobals) * (size_t)M, 128, b->image_bytes,
-                       sizeof(RenderArgs) * (size_t)M, sizeof(WNode) * (size_t)(NI + M), sizeof(uint2) * (size_t)N};
+                       sizeof(RenderArgs) * (size_t)M, sizeof(WNode) * (size_t)(NI + 1), sizeof(uint4) * (size_t)N,
+                       sizeof(int2) * (size_t)(NI > 0 ? NI : 1)};
   const int K = sizeof(sz) / sizeof(sz[0]);
   std::vector<size_t> off(K);
   size_t total = 0;
@@ -314,7 +315,9 @@ crt_status crt_batch_create(const crt_mesh_desc* meshes, const crt_batch_view* v
   b->image = (uint8_t*)at(18);
   b->args = (RenderArgs*)at(19);
   bb.wnodes = (WNode*)at(20);
-  bb.arrivals = (uint2*)at(21);
+  bb.arrivals = (uint4*)at(21);
+  bb.nbox = (float4*)at(14);
+  bb.kids = (int2*)at(22);
   BatchView& v = b->v;
   b->d_item_off = d_ioff;
   v.M = M, v.tri_off = d_toff;
@@ -496,45 +499,26 @@ crt_status crt_batch_export(crt_batch* b, int32_t m, float* scene_box, int32_t* 
     std::memcpy(&f, &bits, 4);
     return f;
   };
-  std::vector<uint32_t> hk(n), hv(n), par_i(n > 1 ? n - 1 : 0), par_l(n);
+  std::vector<uint32_t> hk(n), hv(n), par(nn);
+  std::vector<LeafTri> lf(n);
   std::vector<WNode> wn(n > 1 ? n - 1 : 0);
-  WNode wroot;
   CRT_CUDA(cudaMemcpy(hk.data(), b->b.keys_b + t0, 4 * (size_t)n, cudaMemcpyDeviceToHost), "download");
   CRT_CUDA(cudaMemcpy(hv.data(), b->b.vals_a + t0, 4 * (size_t)n, cudaMemcpyDeviceToHost), "download");
-  CRT_CUDA(cudaMemcpy(par_l.data(), b->b.parent + NI + t0, 4 * (size_t)n, cudaMemcpyDeviceToHost), "download");
+  CRT_CUDA(cudaMemcpy(lf.data(), b->b.leaves + t0, sizeof(LeafTri) * (size_t)n, cudaMemcpyDeviceToHost), "download");
   if (n > 1) {
-    CRT_CUDA(cudaMemcpy(par_i.data(), b->b.parent + ib, 4 * (size_t)(n - 1), cudaMemcpyDeviceToHost), "download");
+    CRT_CUDA(cudaMemcpy(par.data() + (n - 1), b->b.parent + NI + t0, 4 * (size_t)n, cudaMemcpyDeviceToHost), "download");
+    CRT_CUDA(cudaMemcpy(par.data(), b->b.parent + ib, 4 * (size_t)(n - 1), cudaMemcpyDeviceToHost), "download");
     CRT_CUDA(cudaMemcpy(wn.data(), b->b.wnodes + ib, sizeof(WNode) * (n - 1), cudaMemcpyDeviceToHost), "download");
-    CRT_CUDA(cudaMemcpy(&wroot, b->b.wnodes + NI + m, sizeof(WNode), cudaMemcpyDeviceToHost), "download");
+    // parent words hold indices into the batch's nodes
+    for (size_t i = 0; i < nn; i++) par[i] = (par[i] & (1u << 31)) | (uint32_t)((int)(par[i] & ((1u << 30) - 1)) - ib);
   }
-  const uint32_t mask = (1u << 30) - 1;
   std::vector<int> n3(3 * nn);
   std::vector<float> nb(6 * nn);
-  auto ref = [n](int code) { return code >= 0 ? code : (n - 1) + ~code; };
-  for (int i = 0; i < n - 1; i++) n3[3 * i] = i == 0 ? -1 : (int)(par_i[i] & mask) - ib;
+  if (!export_tree(n, par.data(), wn.data(), lf.data(), g.root_box, n3.data(), nb.data()))
+    return fail(CRT_CUDA_ERROR, "inconsistent tree");
   for (int k = 0; k < n; k++) {
-    n3[3 * ((n - 1) + k)] = n > 1 ? (int)(par_l[k] & mask) - ib : -1;
     n3[3 * ((n - 1) + k) + 1] = n3[3 * ((n - 1) + k) + 2] = (int)hv[k] - t0;
   }
-  // the children of internal node i sit in the wide node of its parent (the
-  // root's in the mesh's virtual node), slots 2*side(i) and 2*side(i) + 1
-  for (int i = 0; i < n - 1; i++) {
-    const int pl = (int)(par_i[i] & mask) - ib;
-    if (i > 0 && (pl < 0 || pl >= n - 1)) return fail(CRT_CUDA_ERROR, "inconsistent tree");
-    const WNode& gw = i == 0 ? wroot : wn[pl];
-    const int s0 = (i == 0 || (par_i[i] >> 31)) ? 0 : 2;
-    for (int c = 0; c < 2; c++) {
-      const WSlot& q = gw.s[s0 + c];
-      int code;
-      std::memcpy(&code, &q.lo_code.w, 4);
-      const int r = ref(code);
-      if (code == kNoChild || r < 0 || (size_t)r >= nn) return fail(CRT_CUDA_ERROR, "inconsistent tree");
-      n3[3 * i + 1 + c] = r;
-      const float box[6] = {q.lo_code.x, q.lo_code.y, q.lo_code.z, q.hi.x, q.hi.y, q.hi.z};
-      std::memcpy(&nb[6 * (size_t)r], box, sizeof(box));
-    }
-  }
-  std::memcpy(&nb[0], g.root_box, 6 * sizeof(float));
   float box[6];
   for (int k = 0; k < 3; k++) box[k] = ord2f_h(g.bmin[k]), box[3 + k] = ord2f_h(g.bmax[k]);
   std::vector<int32_t> ids_local(n);

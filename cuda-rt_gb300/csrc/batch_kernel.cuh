@@ -5,8 +5,7 @@
 // [tri_off[m], tri_off[m+1]) and internal nodes [tri_off[m] - m,
 // tri_off[m+1] - m - 1)).  Child codes in the wide nodes are local to the
 // mesh, so each mesh's node and leaf ranges are a self-contained tree for the
-// traversal; parent words hold global internal indices; mesh m's virtual
-// wide node (its root's children) is NI + m.
+// traversal; parent words hold global internal indices.
 //
 // k_batch runs the phases below one after another, every block taking part
 // in every phase, with a grid-wide barrier between them (the launch is
@@ -243,23 +242,21 @@ __device__ __noinline__ void ph_hierarchy(const BatchBufs b) {
     b.parent[c1 < 0 ? NI + t0 + split : ib + split] = (uint32_t)gi | kParentLeft | spans;
     b.parent[c2 < 0 ? NI + t0 + split + 1 : ib + split + 1] = (uint32_t)gi | spans;
     b.flags[gi] = 0;
-    const float4 empty = make_float4(0.f, 0.f, 0.f, __int_as_float(kNoChild));
-    if (c1 < 0) __stcg(&b.wnodes[gi].s[1].lo_code, empty);
-    if (c2 < 0) __stcg(&b.wnodes[gi].s[3].lo_code, empty);
   }
 }
 
-// Shared memory of the refit phase: the children's boxes at each block-local
-// node of the chunk (lo xyz, hi xyz) and the nodes' arrival counts.
+// Shared memory of the refit phase: the children's boxes and codes at each
+// block-local node of the chunk and the nodes' arrival counts.
 struct RefitSmem {
-  float box[kRefitBlock][2][6];
+  SlotBox box[kRefitBlock][2];
   int flag[kRefitBlock];
 };
 
 // The climb of one leaf (global sorted position k) through the block-local
 // nodes of its chunk of kRefitBlock leaves (RefitBounds, kernels/bvh.cu:
 // 209-258): the second arrival at a node takes the union; a climb that
-// reaches a node spanning several chunks is handed on.
+// reaches a node spanning several chunks leaves its box (and its children's
+// boxes and codes) in nbox and kids and is handed on.
 __device__ __forceinline__ void refit_leaf(const BatchBufs& b, RefitSmem& sm, int k0, int k) {
   const int N = b.N, NI = b.NI;
   const int tri = (int)ld_in<false>(b.vals_a + k);
@@ -283,6 +280,7 @@ __device__ __forceinline__ void refit_leaf(const BatchBufs& b, RefitSmem& sm, in
     return;
   }
   const int root = t0 - m;
+  SlotBox* nbox = reinterpret_cast<SlotBox*>(b.nbox);
   uint32_t w = ld_in<false>(b.parent + NI + k);
   int xc = ~(k - t0);  // codes are local to the mesh
   for (int level = 0;; level++) {
@@ -291,30 +289,34 @@ __device__ __forceinline__ void refit_leaf(const BatchBufs& b, RefitSmem& sm, in
       atomicOr(&b.g[m].err, kErrStack);
       return;
     }
+    if (w & kParentSpans) {  // the climb continues in the refit-top phase
+      if (xc >= 0) {
+        const int x = root + xc, sl = t0 + xc - k0;
+        store_box(nbox + x, SlotBox{make_float4(lo[0], lo[1], lo[2], 0.f), make_float4(hi[0], hi[1], hi[2], 0.f)});
+        int kid[2];
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+          const SlotBox& q = sm.box[sl][side];
+          kid[side] = __float_as_int(q.hi.w);
+          if (kid[side] >= 0) store_box(nbox + root + kid[side], q);
+        }
+        __stcg(b.kids + x, make_int2(kid[0], kid[1]));
+      }
+      b.arrivals[atomicAdd(b.counters + 6, 1u)] = make_uint4(w, (uint32_t)m, (uint32_t)xc, 0u);
+      return;
+    }
     const uint32_t wn = (p == root) ? 0u : ld_in<false>(b.parent + p);
     const bool is_left = (w & kParentLeft) != 0;
-    const int gp = (p == root) ? NI + m : (int)(wn & kParentMask);
-    const bool p_left = (p == root) || (wn & kParentLeft) != 0;
-    if (p != root && (gp < root || gp >= root + n - 1)) {  // only a corrupt tree gets here
-      atomicOr(&b.g[m].err, kErrStack);
-      return;
-    }
-    put_wide(b.wnodes, xc, is_left, p, gp, p_left, lo, hi);
-    if (!(w & kParentSpans)) {
-      const int sl = p + m - k0;  // global leaf position of the node's index, within this chunk
-      float* mine = sm.box[sl][is_left ? 0 : 1];
-#pragma unroll
-      for (int q = 0; q < 3; q++) mine[q] = lo[q], mine[3 + q] = hi[q];
-      __threadfence_block();
-      if (atomicAdd(&sm.flag[sl], 1) == 0) return;  // first arrival
-      __threadfence_block();
-      const float* o = sm.box[sl][is_left ? 1 : 0];
-#pragma unroll
-      for (int q = 0; q < 3; q++) lo[q] = fminf(lo[q], o[q]), hi[q] = fmaxf(hi[q], o[3 + q]);
-    } else {  // spanning node: the climb continues in the refit-top phase
-      b.arrivals[atomicAdd(b.counters + 6, 1u)] = make_uint2(w, (uint32_t)m);
-      return;
-    }
+    const int sl = p + m - k0;  // global leaf position of the node's index, within this chunk
+    SlotBox& mine = sm.box[sl][is_left ? 0 : 1];
+    mine.lo = make_float4(lo[0], lo[1], lo[2], 0.f);
+    mine.hi = make_float4(hi[0], hi[1], hi[2], __int_as_float(xc));
+    __threadfence_block();
+    if (atomicAdd(&sm.flag[sl], 1) == 0) return;  // first arrival
+    __threadfence_block();
+    const float4 ol = sm.box[sl][is_left ? 1 : 0].lo, oh = sm.box[sl][is_left ? 1 : 0].hi;
+    lo[0] = fminf(lo[0], ol.x), lo[1] = fminf(lo[1], ol.y), lo[2] = fminf(lo[2], ol.z);
+    hi[0] = fmaxf(hi[0], oh.x), hi[1] = fmaxf(hi[1], oh.y), hi[2] = fmaxf(hi[2], oh.z);
     if (p == root) {
 #pragma unroll
       for (int q = 0; q < 3; q++) b.g[m].root_box[q] = lo[q], b.g[m].root_box[3 + q] = hi[q];
@@ -327,7 +329,8 @@ __device__ __forceinline__ void refit_leaf(const BatchBufs& b, RefitSmem& sm, in
 
 // The block takes chunks of kRefitBlock sorted leaves in turn; each thread
 // climbs from kRefitBlock / blockDim.x leaves of the chunk, one after
-// another (a climb never waits: the first arrival at a node stops).
+// another (a climb never waits: the first arrival at a node stops), then the
+// block writes the wide nodes of the chunk's block-local nodes.
 __device__ __noinline__ void ph_refit(const BatchBufs b, RefitSmem& sm) {
   const int N = b.N;
   const int chunks = (N + kRefitBlock - 1) / kRefitBlock;
@@ -338,66 +341,72 @@ __device__ __noinline__ void ph_refit(const BatchBufs b, RefitSmem& sm) {
     for (int i = threadIdx.x; i < kRefitBlock; i += blockDim.x)
       if (k0 + i < N) refit_leaf(b, sm, k0, k0 + i);
     __syncthreads();
+    for (int i = threadIdx.x; i < kRefitBlock; i += blockDim.x)
+      if (sm.flag[i] == 2) {
+        // node index = leaf position - mesh number; its mesh is that of the leaf there
+        const int m = __ldg(b.mesh_of + (int)ld_in<false>(b.vals_a + k0 + i));
+        const int t0 = __ldg(b.tri_off + m);
+        write_wide(b.wnodes + (k0 + i - m), sm.box[i][0], sm.box[i][1],
+                   [&](int c, int side) { return sm.box[min(max(t0 + c - k0, 0), kRefitBlock - 1)][side]; });
+      }
+    __syncthreads();
   }
 }
 
-// The handed-on climbs through the spanning nodes: each arrival meets its
-// sibling at gpu scope (a release/acquire add on the node's flag, whose
-// parity tells the second arrival), which takes the union and climbs on.
+// The handed-on climbs through the spanning nodes: each arrival leaves its
+// code, meets its sibling at gpu scope (a release/acquire add on the node's
+// flag, whose parity tells the second arrival), and the second one takes the
+// union, writes the node's wide node and climbs on.
 __device__ __noinline__ void ph_refit_top(const BatchBufs b) {
   const int M = b.M, NI = b.NI;
   const unsigned count = ld_in<false>(b.counters + 6);
-  WNode* wnodes = b.wnodes;
+  SlotBox* nbox = reinterpret_cast<SlotBox*>(b.nbox);
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    const uint2 arr = b.arrivals[i];
+    const uint4 arr = __ldcg(b.arrivals + i);
     const int m = (int)arr.y;
     if (m < 0 || m >= M) continue;  // only a corrupt arrival gets here
     const int t0 = __ldg(b.tri_off + m), n = __ldg(b.tri_off + m + 1) - t0, root = t0 - m;
     uint32_t w = arr.x;
-    int p = (int)(w & kParentMask);
-    if (p < root || p >= root + n - 1) {
-      atomicOr(&b.g[m].err, kErrStack);
-      continue;
-    }
-    uint32_t wn = (p == root) ? 0u : ld_in<false>(b.parent + p);
-    bool is_left = (w & kParentLeft) != 0;
-    int gp = (p == root) ? NI + m : (int)(wn & kParentMask);
-    bool p_left = (p == root) || (wn & kParentLeft) != 0;
-    if (p != root && (gp < root || gp >= root + n - 1)) {
-      atomicOr(&b.g[m].err, kErrStack);
-      continue;
-    }
-    float lo[3], hi[3];
-    {
-      const WSlot* q = wnodes[gp].s + (p_left ? 0 : 2) + (is_left ? 0 : 1);
-      const float4 a = __ldcg(&q->lo_code), bb = __ldcg(&q->hi);
-      lo[0] = a.x, lo[1] = a.y, lo[2] = a.z, hi[0] = bb.x, hi[1] = bb.y, hi[2] = bb.z;
-    }
+    int xc = (int)arr.z;
+    auto box_of = [&](int code) {  // the box of a node of this mesh, its code in hi.w
+      SlotBox q = code < 0 ? leaf_box(b.leaves, t0 + ~code) : load_box(nbox + root + code);
+      q.hi.w = __int_as_float(code);
+      return q;
+    };
+    auto valid = [&](int code) { return code < 0 ? ~code < n : code < n - 1; };
     for (int level = 0;; level++) {
-      const uint32_t wn_next = (p == root) ? 0u : __ldcg(b.parent + gp);
+      const int p = (int)(w & kParentMask);
+      if (level >= kStackSize || p < root || p >= root + n - 1 || !valid(xc)) {  // only a corrupt tree gets here
+        atomicOr(&b.g[m].err, kErrStack);
+        break;
+      }
+      const uint32_t wn = (p == root) ? 0u : __ldcg(b.parent + p);
+      const bool is_left = (w & kParentLeft) != 0;
+      __stcg(reinterpret_cast<int*>(b.kids + p) + (is_left ? 0 : 1), xc);
       if ((atomic_add_acq_rel(b.flags + p, 1) & 1) == 0) break;  // first arrival
-      sibling_box(wnodes, gp, p_left, is_left, lo, hi);
+      const int2 kid = __ldcg(b.kids + p);
+      if (!valid(kid.x) || !valid(kid.y)) {  // only a corrupt tree gets here
+        atomicOr(&b.g[m].err, kErrStack);
+        break;
+      }
+      const SlotBox left = box_of(kid.x), right = box_of(kid.y);
+      write_wide(b.wnodes + p, left, right, [&](int c, int side) {
+        const int2 g = __ldcg(b.kids + root + c);
+        const int code = side ? g.y : g.x;
+        return box_of(valid(code) ? code : -1);
+      });
+      const float4 lo = make_float4(fminf(left.lo.x, right.lo.x), fminf(left.lo.y, right.lo.y),
+                                    fminf(left.lo.z, right.lo.z), 0.f);
+      const float4 hi = make_float4(fmaxf(left.hi.x, right.hi.x), fmaxf(left.hi.y, right.hi.y),
+                                    fmaxf(left.hi.z, right.hi.z), 0.f);
       if (p == root) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) b.g[m].root_box[q] = lo[q], b.g[m].root_box[3 + q] = hi[q];
+        float* r = b.g[m].root_box;
+        r[0] = lo.x, r[1] = lo.y, r[2] = lo.z, r[3] = hi.x, r[4] = hi.y, r[5] = hi.z;
         break;
       }
-      const int xc = p - root;
+      store_box(nbox + p, SlotBox{lo, hi});
+      xc = p - root;
       w = wn;
-      p = (int)(w & kParentMask);
-      if (level >= kStackSize || p < root || p >= root + n - 1) {
-        atomicOr(&b.g[m].err, kErrStack);
-        break;
-      }
-      wn = wn_next;
-      is_left = (w & kParentLeft) != 0;
-      gp = (p == root) ? NI + m : (int)(wn & kParentMask);
-      p_left = (p == root) || (wn & kParentLeft) != 0;
-      if (p != root && (gp < root || gp >= root + n - 1)) {
-        atomicOr(&b.g[m].err, kErrStack);
-        break;
-      }
-      put_wide(wnodes, xc, is_left, p, gp, p_left, lo, hi);
     }
   }
 }

@@ -11,7 +11,8 @@
 //                  look-back, when the tiles do not all fit at once)
 //   k_hierarchy    Karras split search, one thread per internal node
 //   k_refit        atomic bottom-up refit, one climber per leaf; it also
-//                  writes the leaf triangles in sorted order for traversal
+//                  writes the leaf triangles in sorted order and the wide
+//                  nodes for traversal
 // Triangle boxes are never stored: each stage that needs one recomputes it
 // from the three vertices (L2-resident for the sizes this targets).
 #include <cstdio>
@@ -336,11 +337,9 @@ __global__ void __launch_bounds__(TH, 1) k_sort_coop(uint32_t* keys_a, uint32_t*
 
 // BuildHierarchy (kernels/bvh.cu:164-207) with FindSpan (bvh.cu:100-133) and
 // FindSplit (bvh.cu:134-162): one thread per internal node writes its
-// children's parent words and lists its spanning children for
-// k_refit_spans (the child codes and boxes reach the wide nodes through the
-// refit, which relies on the empty odd slot marked here beside a leaf
-// child).  Every probe of a node
-// whose span is at most kShortSpan leaves lies within kShortSpan of the node,
+// children's parent words and its split, and lists itself for k_refit_spans
+// when it spans refit blocks (child codes and boxes reach the wide nodes
+// through the refit).  Every probe of a node whose span is at most kShortSpan leaves lies within kShortSpan of the node,
 // so a block first stages the codes of its nodes +- kShortSpan in shared
 // memory (one coalesced load) and searches there.  A node whose span turns
 // out longer (the nodes near the root, whose binary searches are the longest
@@ -361,7 +360,7 @@ __device__ __forceinline__ int kdelta_s(const uint32_t* s_c, int w0, int n, uint
 }
 
 __global__ void __launch_bounds__(kHierThreads) k_hierarchy(const uint32_t* __restrict__ codes, int n,
-                                                            uint32_t* __restrict__ parent, WNode* __restrict__ wnodes,
+                                                            uint32_t* __restrict__ parent, int* __restrict__ splits,
                                                             uint4* __restrict__ spans, unsigned* nspan) {
   __shared__ uint32_t s_c[kHierWindow];
   pdl_wait();
@@ -423,32 +422,22 @@ __global__ void __launch_bounds__(kHierThreads) k_hierarchy(const uint32_t* __re
   }
   const int c1 = (split == lo) ? ~split : split;
   const int c2 = (split + 1 == hi) ? ~(split + 1) : split + 1;
+  const bool crosses = act && lo / kRefitBlock != hi / kRefitBlock;
   if (spans) {
-    // the spanning children (internal nodes whose leaf range crosses a
-    // kRefitBlock boundary) join the list k_refit_spans works through:
-    // (node, first leaf, last leaf, parent word)
-    const bool s1 = act && c1 >= 0 && lo / kRefitBlock != split / kRefitBlock;
-    const bool s2 = act && c2 >= 0 && (split + 1) / kRefitBlock != hi / kRefitBlock;
-    const uint32_t m1 = __ballot_sync(0xffffffffu, s1), m2 = __ballot_sync(0xffffffffu, s2);
-    if (m1 | m2) {
+    const uint32_t m = __ballot_sync(0xffffffffu, crosses);
+    if (m) {
       unsigned base = 0;
-      if (lane == 0) base = atomicAdd(nspan, (unsigned)(__popc(m1) + __popc(m2)));
+      if (lane == 0) base = atomicAdd(nspan, (unsigned)__popc(m));
       base = __shfl_sync(0xffffffffu, base, 0);
-      const uint32_t lt = lanemask_lt();
-      const uint32_t pw = (uint32_t)i | ((lo / kRefitBlock != hi / kRefitBlock) ? kParentSpans : 0u);
-      if (s1) spans[base + __popc(m1 & lt)] = make_uint4((uint32_t)c1, (uint32_t)lo, (uint32_t)split, pw | kParentLeft);
-      if (s2)
-        spans[base + __popc(m1) + __popc(m2 & lt)] = make_uint4((uint32_t)c2, (uint32_t)(split + 1), (uint32_t)hi, pw);
+      if (crosses)
+        spans[base + __popc(m & lanemask_lt())] = make_uint4((uint32_t)i, (uint32_t)lo, (uint32_t)hi, (uint32_t)split);
     }
   }
   if (!act) return;
-  const uint32_t spanbit = (lo / kRefitBlock != hi / kRefitBlock) ? kParentSpans : 0u;
+  if (splits) splits[i] = split;
+  const uint32_t spanbit = crosses ? kParentSpans : 0u;
   parent[c1 < 0 ? (n - 1) + split : split] = (uint32_t)i | kParentLeft | spanbit;
   parent[c2 < 0 ? (n - 1) + split + 1 : split + 1] = (uint32_t)i | spanbit;
-  // a leaf child takes one slot of this node's wide node: mark the other empty
-  const float4 empty = make_float4(0.f, 0.f, 0.f, __int_as_float(kNoChild));
-  if (c1 < 0) wnodes[i].s[1].lo_code = empty;
-  if (c2 < 0) wnodes[i].s[3].lo_code = empty;
 }
 
 // Box helpers: six floats (lo xyz, hi xyz) at 8-byte aligned addresses,
@@ -466,104 +455,139 @@ __device__ __forceinline__ void box_store6(float* q, const float b[6]) {
   __stcg(d + 2, make_float2(b[4], b[5]));
 }
 
-// The boxes of the spanning nodes (leaf ranges over several refit blocks).
-// Each is the union of its leaves' boxes, and its leaf range [lo, hi] is
-// known from the split search, so no climb is needed: the box is the union
-// of the boxes of leaves lo..end of lo's block (suf[lo]), of the blocks in
-// between (suf at a block's first leaf, or gbox for whole groups of
-// kSpanGroup blocks) and of leaves start of hi's block..hi (pre[hi]), all
-// written by k_refit.  (lo
-// starts the leftmost maximal block-local node under the spanning node,
+// The wide nodes of the spanning nodes (leaf ranges over several refit
+// blocks).  The box of a leaf range is the union of its leaves' boxes, and the
+// split search gives every range, so no climb is needed.  For each listed node
+// (node, first leaf, last leaf, split) kSpanLanes lanes work out each of its
+// four slots: the box of a leaf or of a block-local node was left by k_refit
+// (leaves, nbox); that of a range over several blocks is the union of the
+// boxes of leaves lo..end of lo's block (suf[lo]), of the blocks in between
+// (suf at a block's first leaf, or gbox for whole groups of kSpanGroup blocks)
+// and of leaves start of hi's block..hi (pre[hi]), all written by k_refit.
+// (lo starts the leftmost maximal block-local node under the spanning node,
 // which is a left child of a spanning node, and hi ends the rightmost one, a
 // right child: k_refit writes suf and pre at both ends of every such node.)
-// kSpanLanes lanes per listed node share the blocks and groups in between;
-// the item after the list is the root.  min/max are exact, so the boxes
-// equal those of the reference's climb.
+// The root spans whenever there is more than one block; its slots give the
+// root box.  min/max are exact, so the boxes equal those of the reference's
+// climb.
 constexpr int kSpanLanes = 8;
 
-__global__ void __launch_bounds__(256) k_refit_spans(WNode* wnodes, const uint32_t* __restrict__ parent,
-                                                     const uint4* __restrict__ spans, const float* suf,
-                                                     const float* pre, const int* gbox, int n, SceneGlobals* g) {
+__global__ void __launch_bounds__(256) k_refit_spans(WNode* wnodes, const uint4* __restrict__ spans,
+                                                     const int* __restrict__ splits, const LeafTri* leaves,
+                                                     const SlotBox* nbox, const float* suf, const float* pre,
+                                                     const int* gbox, int n, SceneGlobals* g) {
   pdl_wait();
   pdl_launch_dependents();
+  const unsigned full = 0xffffffffu;
   const unsigned count = *(volatile unsigned*)&g->nspan;
-  const int sub = threadIdx.x & (kSpanLanes - 1);
-  const unsigned groups = (gridDim.x * blockDim.x) / kSpanLanes;
-  const unsigned first = (blockIdx.x * blockDim.x + threadIdx.x) / kSpanLanes;
-  // every lane of a warp runs the same number of rounds (the shuffles below)
-  const unsigned rounds = (count + 1 + groups - 1) / groups;
-  for (unsigned rnd = 0; rnd < rounds; rnd++) {
-    const unsigned item = first + rnd * groups;
-    const bool live = item <= count;
-    const bool root = item == count;
-    uint4 e = make_uint4(0u, 0u, (uint32_t)(n - 1), 0u);
-    if (live && !root) e = __ldg(spans + item);
-    const int lo = (int)e.y, hi = (int)e.z;
-    bool ok = live;
-    if (live && !root && ((unsigned)lo >= (unsigned)n || (unsigned)hi >= (unsigned)n ||
-                          lo / kRefitBlock >= hi / kRefitBlock)) {
-      if (sub == 0) atomicOr(&g->err, kErrStack);  // only a corrupt list gets here
-      ok = false;
+  const int lane = threadIdx.x & 31, sub = lane & (kSpanLanes - 1), slot = lane / kSpanLanes;
+  const unsigned warps = (gridDim.x * blockDim.x) / 32;
+  for (unsigned item = (blockIdx.x * blockDim.x + threadIdx.x) / 32; item < count; item += warps) {
+    const uint4 e = __ldg(spans + item);
+    const int x = (int)e.x, lo = (int)e.y, hi = (int)e.z, split = (int)e.w;
+    if (x < 0 || x >= n - 1 || lo < 0 || hi >= n || split < lo || split >= hi) {  // only a corrupt list gets here
+      if (lane == 0) atomicOr(&g->err, kErrStack);
+      continue;
     }
-    // blocks strictly between the ends (the root: all): [b0, h) and [t, b1)
-    // one by one, the whole groups in [h, t) from gbox
-    const int b0 = root ? 0 : lo / kRefitBlock + 1;
-    int b1 = root ? (n - 1) / kRefitBlock + 1 : hi / kRefitBlock;
-    int h = min(b1, (b0 + kSpanGroup - 1) / kSpanGroup * kSpanGroup);
-    int t = max(h, b1 / kSpanGroup * kSpanGroup);
-    if (!ok) h = t = b1 = b0;
-    const int nh = h - b0, ng = (t - h) / kSpanGroup, nt = b1 - t, total = nh + ng + nt;
-    float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    for (int j = sub; j < total; j += kSpanLanes) {
-      if (j >= nh && j < nh + ng) {
-        const int* q = gbox + 6 * (size_t)(h / kSpanGroup + j - nh);
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-          b[c] = fminf(b[c], ord2f(__ldcg(q + c))), b[3 + c] = fmaxf(b[3 + c], ord2f(__ldcg(q + 3 + c)));
+    // this slot's leaf range [a, b] and code
+    int a = slot < 2 ? lo : split + 1, b = slot < 2 ? split : hi;
+    int code = a == b ? ((slot & 1) ? kNoChild : ~a) : (slot < 2 ? split : split + 1);
+    if (a != b) {  // an internal child: its own children
+      const int s2 = __ldg(splits + code);
+      if (s2 < a || s2 >= b) {  // only a corrupt tree gets here
+        if (sub == 0) atomicOr(&g->err, kErrStack);
+        a = b, code = kNoChild;
+      } else if ((slot & 1) == 0) {
+        b = s2;
+        code = a == b ? ~a : s2;
       } else {
-        box_union6(b, suf + 6 * (size_t)kRefitBlock * (size_t)(j < nh ? b0 + j : t + j - nh - ng));
+        a = s2 + 1;
+        code = a == b ? ~a : s2 + 1;
       }
     }
-    if (__any_sync(0xffffffffu, total > 0)) {
+    float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    const int blk = a / kRefitBlock, last = b / kRefitBlock;
+    if (code != kNoChild) {
+      if (blk == last) {
+        if (sub == 0) {
+          const SlotBox q = code < 0 ? leaf_box(leaves, a) : load_box(nbox + code);
+          v[0] = q.lo.x, v[1] = q.lo.y, v[2] = q.lo.z, v[3] = q.hi.x, v[4] = q.hi.y, v[5] = q.hi.z;
+        }
+      } else {
+        // blocks strictly between the ends: [b0, h) and [t, b1) one by one,
+        // the whole groups in [h, t) from gbox
+        const int b0 = blk + 1, b1 = last;
+        const int h = min(b1, (b0 + kSpanGroup - 1) / kSpanGroup * kSpanGroup);
+        const int t = max(h, b1 / kSpanGroup * kSpanGroup);
+        const int nh = h - b0, ng = (t - h) / kSpanGroup, nt = b1 - t, total = nh + ng + nt;
+        if (sub == 0) box_union6(v, suf + 6 * (size_t)a);
+        if (sub == 1) box_union6(v, pre + 6 * (size_t)b);
+        for (int j = (sub + kSpanLanes - 2) % kSpanLanes; j < total; j += kSpanLanes) {
+          if (j >= nh && j < nh + ng) {
+            const int* q = gbox + 6 * (size_t)(h / kSpanGroup + j - nh);
 #pragma unroll
-      for (int o = kSpanLanes / 2; o > 0; o >>= 1) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-          b[q] = fminf(b[q], __shfl_xor_sync(0xffffffffu, b[q], o));
-          b[3 + q] = fmaxf(b[3 + q], __shfl_xor_sync(0xffffffffu, b[3 + q], o));
+            for (int c = 0; c < 3; c++)
+              v[c] = fminf(v[c], ord2f(__ldcg(q + c))), v[3 + c] = fmaxf(v[3 + c], ord2f(__ldcg(q + 3 + c)));
+          } else {
+            box_union6(v, suf + 6 * (size_t)kRefitBlock * (size_t)(j < nh ? b0 + j : t + j - nh - ng));
+          }
         }
       }
     }
-    if (!ok || sub != 0) continue;
-    if (root) {
 #pragma unroll
-      for (int q = 0; q < 6; q++) g->root_box[q] = b[q];
-      continue;
+    for (int o = kSpanLanes / 2; o > 0; o >>= 1) {
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        v[q] = fminf(v[q], __shfl_xor_sync(full, v[q], o));
+        v[3 + q] = fmaxf(v[3 + q], __shfl_xor_sync(full, v[3 + q], o));
+      }
     }
-    box_union6(b, suf + 6 * (size_t)lo);
-    box_union6(b, pre + 6 * (size_t)hi);
-    const int x = (int)e.x, p = (int)(e.w & kParentMask);
-    const uint32_t wn = (p == 0) ? 0u : __ldg(parent + p);
-    const int gp = (p == 0) ? n - 1 : (int)(wn & kParentMask);
-    if (x <= 0 || x >= n - 1 || p >= n - 1 || (p != 0 && gp >= n - 1)) {  // only a corrupt tree gets here
-      atomicOr(&g->err, kErrStack);
-      continue;
+    // the node's box (an empty slot's is the empty box), then one axis per
+    // lane: the bytes of the lane's own slot, joined over the slots
+    float u[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      u[q] = v[q];
+#pragma unroll
+      for (int o = kSpanLanes; o < 32; o <<= 1) {
+        const float y = __shfl_xor_sync(full, u[q], o);
+        u[q] = q < 3 ? fminf(u[q], y) : fmaxf(u[q], y);
+      }
     }
-    const float lo3[3] = {b[0], b[1], b[2]}, hi3[3] = {b[3], b[4], b[5]};
-    put_wide(wnodes, x, (e.w & kParentLeft) != 0, p, gp, (p == 0) || (wn & kParentLeft) != 0, lo3, hi3);
+    const int axis = min(sub, 2);
+    const float og = axis == 0 ? u[0] : (axis == 1 ? u[1] : u[2]), hm = axis == 0 ? u[3] : (axis == 1 ? u[4] : u[5]);
+    const float bl = axis == 0 ? v[0] : (axis == 1 ? v[1] : v[2]), bh = axis == 0 ? v[3] : (axis == 1 ? v[4] : v[5]);
+    const QAxis qa = q_axis(og, hm);
+    uint32_t ql = (code == kNoChild ? 255u : q_lo(qa, bl)) << (8 * slot);
+    uint32_t qh = (code == kNoChild ? 0u : q_hi(qa, bh)) << (8 * slot);
+#pragma unroll
+    for (int o = kSpanLanes; o < 32; o <<= 1) {
+      ql |= __shfl_xor_sync(full, ql, o);
+      qh |= __shfl_xor_sync(full, qh, o);
+    }
+    WNode* w = wnodes + x;
+    if (slot == 0 && sub < 3) w->o[axis] = qa.o, w->s15[axis] = qa.s15, w->lo[axis] = ql, w->hi[axis] = qh;
+    if (sub == 3) w->code[slot] = code;
+    if (x == 0 && lane == 0) {
+#pragma unroll
+      for (int q = 0; q < 6; q++) g->root_box[q] = u[q];
+    }
   }
 }
 
-__global__ void __launch_bounds__(kRefitBlock, 4) k_refit(const float* __restrict__ V, const int* __restrict__ vidx,
+// (Three blocks per SM, 40 registers: 1,003,520 triangles build in 216.5 us;
+// with two 221.1 us, with four, which spill, 230.1 us.  220.5 us when every
+// climber wrote its slots of two 128-byte wide nodes at each step.)
+__global__ void __launch_bounds__(kRefitBlock, 3) k_refit(const float* __restrict__ V, const int* __restrict__ vidx,
                                                        const uint32_t* __restrict__ ids, int n,
                                                        WNode* wnodes, LeafTri* __restrict__ leaves,
                                                        const uint32_t* __restrict__ parent, float* __restrict__ suf,
                                                        float* __restrict__ pre, int* __restrict__ gbox,
-                                                       SceneGlobals* g) {
-  // children's boxes at each block-local node (lo, hi); lo.w: the leaf-range
-  // end the first arrival brings (its first leaf if it is the left child,
-  // else its last)
-  __shared__ float4 s_box[kRefitBlock][2][2];
+                                                       SlotBox* __restrict__ nbox, SceneGlobals* g) {
+  // children's boxes at each block-local node; lo.w: the leaf-range end the
+  // first arrival brings (its first leaf if it is the left child, else its
+  // last), hi.w: the child's code
+  __shared__ float4 s_lo[2][kRefitBlock], s_hi[2][kRefitBlock];
   __shared__ int s_flag[kRefitBlock];
   // the block's maximal block-local nodes (their parents span): box, and
   // first / last leaf in lo.w / hi.w
@@ -619,49 +643,48 @@ __global__ void __launch_bounds__(kRefitBlock, 4) k_refit(const float* __restric
           atomicOr(&g->err, kErrStack);
           break;
         }
-        const uint32_t wn = (p == 0) ? 0u : __ldg(parent + p);  // next step's word, issued early
-        const bool is_left = (w & kParentLeft) != 0;
-        const int gp = (p == 0) ? n - 1 : (int)(wn & kParentMask);
-        const bool p_left = (p == 0) || (wn & kParentLeft) != 0;
-        if (gp >= n - 1 && p != 0) {  // only a corrupt tree gets here
-          atomicOr(&g->err, kErrStack);
-          break;
-        }
-        put_wide(wnodes, xc, is_left, p, gp, p_left, lo, hi);
-        if (!(w & kParentSpans)) {  // both arrivals are threads of this block
-          const int sl = p - k0;
-          if ((unsigned)sl >= (unsigned)kRefitBlock) {  // only a corrupt tree gets here
-            atomicOr(&g->err, kErrStack);
-            break;
-          }
-          float4* mine = s_box[sl][is_left ? 0 : 1];
-          mine[0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(is_left ? l : r));
-          mine[1] = make_float4(hi[0], hi[1], hi[2], 0.f);
-          __threadfence_block();
-          // the first arrival stops; only the second climbs on (so a corrupt
-          // tree cannot make a climb loop: each slot lets one climber through)
-          const int arrived = atomicAdd(&s_flag[sl], 1);
-          if (arrived != 1) {
-            if (arrived != 0) atomicOr(&g->err, kErrStack);
-            break;
-          }
-          __threadfence_block();
-          const float4* o = s_box[sl][is_left ? 1 : 0];
-          const float4 ol = o[0], oh = o[1];
-          lo[0] = fminf(lo[0], ol.x), lo[1] = fminf(lo[1], ol.y), lo[2] = fminf(lo[2], ol.z);
-          hi[0] = fmaxf(hi[0], oh.x), hi[1] = fmaxf(hi[1], oh.y), hi[2] = fmaxf(hi[2], oh.z);
-          if (is_left)
-            r = __float_as_int(ol.w);
-          else
-            l = __float_as_int(ol.w);
-        } else {
-          // the parent spans: k_refit_spans finds its box from the block boxes
-          // and the edge boxes written below
+        if (w & kParentSpans) {
+          // the parent spans: k_refit_spans finds its slots from the block
+          // boxes, the edge boxes written below and these nodes' boxes
           top = atomicAdd(&s_ntop, 1);
           s_top[top][0] = make_float4(lo[0], lo[1], lo[2], __int_as_float(l));
           s_top[top][1] = make_float4(hi[0], hi[1], hi[2], __int_as_float(r));
+          if (xc >= 0) {
+            store_box(nbox + xc, SlotBox{make_float4(lo[0], lo[1], lo[2], 0.f), make_float4(hi[0], hi[1], hi[2], 0.f)});
+#pragma unroll
+            for (int side = 0; side < 2; side++) {
+              const SlotBox q{s_lo[side][xc - k0], s_hi[side][xc - k0]};
+              const int c = __float_as_int(q.hi.w);
+              if (c >= 0) store_box(nbox + c, q);
+            }
+          }
           break;
         }
+        const uint32_t wn = (p == 0) ? 0u : __ldg(parent + p);  // next step's word, issued early
+        const bool is_left = (w & kParentLeft) != 0;
+        const int sl = p - k0;  // both arrivals are threads of this block
+        if ((unsigned)sl >= (unsigned)kRefitBlock) {  // only a corrupt tree gets here
+          atomicOr(&g->err, kErrStack);
+          break;
+        }
+        s_lo[is_left ? 0 : 1][sl] = make_float4(lo[0], lo[1], lo[2], __int_as_float(is_left ? l : r));
+        s_hi[is_left ? 0 : 1][sl] = make_float4(hi[0], hi[1], hi[2], __int_as_float(xc));
+        __threadfence_block();
+        // the first arrival stops; only the second climbs on (so a corrupt
+        // tree cannot make a climb loop: each slot lets one climber through)
+        const int arrived = atomicAdd(&s_flag[sl], 1);
+        if (arrived != 1) {
+          if (arrived != 0) atomicOr(&g->err, kErrStack);
+          break;
+        }
+        __threadfence_block();
+        const float4 ol = s_lo[is_left ? 1 : 0][sl], oh = s_hi[is_left ? 1 : 0][sl];
+        lo[0] = fminf(lo[0], ol.x), lo[1] = fminf(lo[1], ol.y), lo[2] = fminf(lo[2], ol.z);
+        hi[0] = fmaxf(hi[0], oh.x), hi[1] = fmaxf(hi[1], oh.y), hi[2] = fmaxf(hi[2], oh.z);
+        if (is_left)
+          r = __float_as_int(ol.w);
+        else
+          l = __float_as_int(ol.w);
         if (p == 0) {
 #pragma unroll
           for (int q = 0; q < 3; q++) g->root_box[q] = lo[q], g->root_box[3 + q] = hi[q];
@@ -672,10 +695,17 @@ __global__ void __launch_bounds__(kRefitBlock, 4) k_refit(const float* __restric
       }
     }
   }
+  __syncthreads();
+  // the wide nodes of the block-local nodes, one thread each
+  if (s_flag[threadIdx.x] == 2)
+    write_wide(wnodes + k, SlotBox{s_lo[0][threadIdx.x], s_hi[0][threadIdx.x]},
+               SlotBox{s_lo[1][threadIdx.x], s_hi[1][threadIdx.x]}, [&](int c, int side) {
+                 const int j = min(max(c - k0, 0), kRefitBlock - 1);  // (a child of a block-local node is one too)
+                 return SlotBox{s_lo[side][j], s_hi[side][j]};
+               });
   // The maximal block-local nodes tile the block's leaves.  Each writes the
   // union of its own and the later ones' boxes at its first leaf (suf) and of
   // the earlier ones' and its own at its last leaf (pre).
-  __syncthreads();
   const int ntop = s_ntop;
   if (top >= 0) {
     const int l = __float_as_int(s_top[top][0].w), r = __float_as_int(s_top[top][1].w);
@@ -763,10 +793,11 @@ static void refit(const MeshBufs& m, const BuildBufs& b, cudaStream_t st) {
   const int n = m.ntri;
   launch_k(true, k_refit, (n + kRefitBlock - 1) / kRefitBlock, kRefitBlock, st, (const float*)m.verts,
            (const int*)m.vidx, (const uint32_t*)b.vals_b, n, b.wnodes, b.leaves, (const uint32_t*)b.parent, b.suf,
-           b.pre, b.gbox, b.g);
+           b.pre, b.gbox, reinterpret_cast<SlotBox*>(b.nbox), b.g);
   if (n > kRefitBlock)
-    launch_k(true, k_refit_spans, num_sms() * 8, 256, st, b.wnodes, (const uint32_t*)b.parent,
-             (const uint4*)b.spans, (const float*)b.suf, (const float*)b.pre, (const int*)b.gbox, n, b.g);
+    launch_k(true, k_refit_spans, num_sms() * 8, 256, st, b.wnodes, (const uint4*)b.spans, (const int*)b.split,
+             (const LeafTri*)b.leaves, reinterpret_cast<const SlotBox*>(b.nbox), (const float*)b.suf,
+             (const float*)b.pre, (const int*)b.gbox, n, b.g);
 }
 
 // Whether the build's sort runs as one cooperative launch (k_sort_coop): its
@@ -831,7 +862,7 @@ cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st)
   }
   if (n >= 2)
     launch_k(true, k_hierarchy, (n - 1 + kHierThreads - 1) / kHierThreads, kHierThreads, st,
-             (const uint32_t*)b.keys_b, n, b.parent, b.wnodes, b.spans, &b.g->nspan);
+             (const uint32_t*)b.keys_b, n, b.parent, b.split, b.spans, &b.g->nspan);
   refit(m, b, st);
   return cudaGetLastError();
 }
@@ -860,10 +891,10 @@ __global__ void __launch_bounds__(256) k_nodes3(const uint32_t* __restrict__ par
 }
 
 cudaError_t launch_stage_hierarchy(const uint32_t* codes, const uint32_t* ids, int n, int* nodes3,
-                                   uint32_t* parent, WNode* wnodes, cudaStream_t st) {
+                                   uint32_t* parent, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (n >= 2)
-    k_hierarchy<<<(n - 1 + kHierThreads - 1) / kHierThreads, kHierThreads, 0, st>>>(codes, n, parent, wnodes,
+    k_hierarchy<<<(n - 1 + kHierThreads - 1) / kHierThreads, kHierThreads, 0, st>>>(codes, n, parent, nullptr,
                                                                                      nullptr, nullptr);
   k_nodes3<<<(2 * n - 1 + 255) / 256, 256, 0, st>>>(parent, ids, n, nodes3);
   return cudaGetLastError();

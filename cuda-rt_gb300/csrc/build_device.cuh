@@ -537,50 +537,135 @@ __device__ __forceinline__ int warp_prefix_end(int limit, Pred pred) {
   return m;
 }
 
+// One axis of a quantised node: o, s15 and the rounding bounds of its origin
+// for the planes of [og, hm] (see WNode).  The quantum is at least 1/250 of
+// the extent and one ulp of the largest coordinate, so that every plane's
+// byte fits (250 + 2 ulps of rounding + 1).
+struct QAxis {
+  float o, s15, up, dn, inv;
+};
+__device__ __forceinline__ QAxis q_axis(float og, float hm) {
+  const float ext = __fmul_ru(__fsub_ru(hm, og), 0.0040000003f);
+  const int ev = (int)((__float_as_uint(ext) + 0x7fffffu) >> 23);
+  const int eu = (int)(__float_as_uint(fmaxf(fabsf(og), fabsf(hm))) >> 23) - 23;
+  const int e = min(max(max(ev, eu), 64), 238);
+  QAxis a;
+  a.s15 = __uint_as_float((uint32_t)(e + 15) << 23);
+  a.inv = __uint_as_float((uint32_t)(254 - e) << 23);
+  a.o = __fsub_rd(og, a.s15);
+  a.up = __fadd_ru(a.o, a.s15);
+  a.dn = __fadd_rd(a.o, a.s15);
+  return a;
+}
+// The plane bytes of x, rounded down or up: adding 2^23 with directed rounding
+// leaves the floor or the ceiling of a value in [0, 255] in the low byte.
+__device__ __forceinline__ uint32_t q_lo(const QAxis& a, float x) {
+  const float v = fminf(fmaxf(__fmul_rd(__fsub_rd(x, a.up), a.inv), 0.f), 255.f);
+  return __float_as_uint(__fadd_rd(v, 8388608.f)) & 255u;
+}
+__device__ __forceinline__ uint32_t q_hi(const QAxis& a, float x) {
+  const float v = fminf(fmaxf(__fmul_ru(__fsub_ru(x, a.dn), a.inv), 0.f), 255.f);
+  return __float_as_uint(__fadd_ru(v, 8388608.f)) & 255u;
+}
+// Eight floats at a 32-byte boundary, in one store.
+__device__ __forceinline__ void st_8(void* p, float4 a, float4 b) {
+  asm volatile("st.global.cg.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+               "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+// The wide node of four slots (code kNoChild: empty).
+__device__ __forceinline__ void pack_wide(WNode* out, const float4 lo[4], const float4 hi[4], const int code[4]) {
+  uint32_t ql[3] = {0, 0, 0}, qh[3] = {0, 0, 0};
+  float o[3], s15[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    float l[4], h[4], og = INFINITY, hm = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      l[j] = k == 0 ? lo[j].x : (k == 1 ? lo[j].y : lo[j].z);
+      h[j] = k == 0 ? hi[j].x : (k == 1 ? hi[j].y : hi[j].z);
+      if (code[j] != kNoChild) og = fminf(og, l[j]), hm = fmaxf(hm, h[j]);
+    }
+    const QAxis a = q_axis(og, hm);
+    o[k] = a.o, s15[k] = a.s15;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const bool e = code[j] == kNoChild;
+      ql[k] |= (e ? 255u : q_lo(a, l[j])) << (8 * j);
+      qh[k] |= (e ? 0u : q_hi(a, h[j])) << (8 * j);
+    }
+  }
+  auto f = [](uint32_t v) { return __uint_as_float(v); };
+  st_8(out, make_float4(o[0], o[1], o[2], s15[0]), make_float4(s15[1], s15[2], f(ql[0]), f(ql[1])));
+  st_8(out->lo + 2, make_float4(f(ql[2]), f(qh[0]), f(qh[1]), f(qh[2])),
+       make_float4(__int_as_float(code[0]), __int_as_float(code[1]), __int_as_float(code[2]), __int_as_float(code[3])));
+}
+
 // RefitBounds (kernels/bvh.cu:209-258): one climber per leaf; at each node the
 // first arrival stops and the second computes the union (bboxunion,
 // bvh.cu:63-69) and climbs on.  min/max are exact, so every schedule gives the
-// reference's boxes.  Every box goes to the wide nodes (WNode): child x (code
-// xc) of binary node p fills slot 2*side(p) + side(x) of the wide node of p's
-// parent gp (for the root, the virtual node past the last internal one), and
-// a leaf child also fills its own slot of p's wide node (the hierarchy marks
-// the odd slot empty).  Codes are rewritten with the boxes, so a refit alone keeps
-// the wide nodes complete, and the children of every node can be read back
-// from its parent's wide node (the export does).
+// reference's boxes.
 //
 // A block owns kRefitBlock consecutive sorted leaves.  A node whose leaf
 // range lies inside that span has both children's climbers in the block, so
 // its two arrivals meet in shared memory with block-scope ordering (most
-// nodes).  The single-scene build (k_refit_spans) then takes each node
-// spanning several blocks as the union of block and block-edge boxes; the
-// batched build meets there too, through a global flag with release/acquire
-// at gpu scope, reading the other child's box from the wide node (global
-// flags count arrivals; each refit adds exactly two per spanning node, so the
-// parity of the old value tells first from second without clearing between
-// refits).  Each climb step needs one dependent load: the parent word (index,
-// side, spanning bit).
-__device__ __forceinline__ void put_wide(WNode* W, int xc, bool x_left, int p, int gp, bool p_left,
-                                         const float lo[3], const float hi[3]) {
-  const float4 a = make_float4(lo[0], lo[1], lo[2], __int_as_float(xc));
-  const float4 b = make_float4(hi[0], hi[1], hi[2], 0.f);
-  if (xc < 0) {  // (the hierarchy marked the odd slot empty)
-    WSlot* q = W[p].s + (x_left ? 0 : 2);
-    __stcg(&q[0].lo_code, a);
-    __stcg(&q[0].hi, b);
+// nodes); each arrival leaves its box and the code of the node it climbed from
+// there.  After the climbs the block writes its wide nodes, one thread per
+// node, from those boxes: every wide node is written once and whole, and the
+// climbs, whose lanes thin out level by level, write nothing.  (With each
+// climber writing its slots of two wide nodes as it went, k_refit took 80 us
+// on 1,003,520 triangles.)  The single-scene build (k_refit_spans) then takes
+// each node spanning several blocks as the union of block and block-edge
+// boxes; the batched build meets there too, through a global flag with
+// release/acquire at gpu scope.  Each climb step needs one dependent load: the
+// parent word (index, side, spanning bit).
+
+// A box and a code as climbers leave them: lo.xyz, hi.xyz, the code in hi.w
+// (and, in the single-scene build, the far end of the node's leaf range in
+// lo.w).
+struct SlotBox {
+  float4 lo, hi;
+};
+
+// The slots of a wide node from its two children: a leaf child takes its even
+// slot itself (the odd one stays empty), an internal child c brings its own
+// children, kids(c, side).
+template <typename Kids>
+__device__ __forceinline__ void write_wide(WNode* out, const SlotBox& left, const SlotBox& right, Kids kids) {
+  float4 lo[4], hi[4];
+  int code[4];
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const SlotBox& ch = side ? right : left;
+    const int c = __float_as_int(ch.hi.w);
+    if (c < 0) {
+      lo[2 * side] = ch.lo, hi[2 * side] = ch.hi, code[2 * side] = c;
+      lo[2 * side + 1] = ch.lo, hi[2 * side + 1] = ch.hi, code[2 * side + 1] = kNoChild;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const SlotBox g = kids(c, j);
+        lo[2 * side + j] = g.lo, hi[2 * side + j] = g.hi, code[2 * side + j] = __float_as_int(g.hi.w);
+      }
+    }
   }
-  WSlot* q = W[gp].s + (p_left ? 0 : 2) + (x_left ? 0 : 1);
-  __stcg(&q->lo_code, a);
-  __stcg(&q->hi, b);
+  pack_wide(out, lo, hi, code);
 }
 
-// The box of the other child of p, from the wide node of p's parent.
-__device__ __forceinline__ void sibling_box(const WNode* W, int gp, bool p_left, bool x_left, float lo[3],
-                                            float hi[3]) {
-  const WSlot* q = W[gp].s + (p_left ? 0 : 2) + (x_left ? 1 : 0);
-  const float4 a = __ldcg(&q->lo_code), b = __ldcg(&q->hi);
-  lo[0] = fminf(lo[0], a.x), lo[1] = fminf(lo[1], a.y), lo[2] = fminf(lo[2], a.z);
-  hi[0] = fmaxf(hi[0], b.x), hi[1] = fmaxf(hi[1], b.y), hi[2] = fmaxf(hi[2], b.z);
+// The box of leaf k from its triangle, as the climbs compute it.
+__device__ __forceinline__ SlotBox leaf_box(const LeafTri* leaves, int k) {
+  const float4* p = reinterpret_cast<const float4*>(leaves + k);
+  const float4 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(p + 2);
+  SlotBox s;
+  s.lo = make_float4(fminf(c.x, fminf(a.x, b.x)), fminf(c.y, fminf(a.y, b.y)), fminf(c.z, fminf(a.z, b.z)), 0.f);
+  s.hi = make_float4(fmaxf(c.x, fmaxf(a.x, b.x)), fmaxf(c.y, fmaxf(a.y, b.y)), fmaxf(c.z, fmaxf(a.z, b.z)), 0.f);
+  return s;
 }
+__device__ __forceinline__ void store_box(SlotBox* p, const SlotBox& b) {
+  __stcg(&p->lo, b.lo);
+  __stcg(&p->hi, b.hi);
+}
+__device__ __forceinline__ SlotBox load_box(const SlotBox* p) { return SlotBox{__ldcg(&p->lo), __ldcg(&p->hi)}; }
 
 }  // namespace
 

@@ -140,6 +140,72 @@ void free_scene(crt_scene* s) {
 namespace crt {
 // Lets entry points in other translation units record their error message.
 void set_last_error(const char* msg) { g_err = msg; }
+
+// A wide node's slot as the traversal reads it contains `box` (exact in
+// double: o is a float, s15 a power of two, the byte term 23 bits).
+static bool slot_contains(const WNode& w, int slot, const float box[6]) {
+  for (int k = 0; k < 3; k++) {
+    const double ql = (w.lo[k] >> (8 * slot)) & 255u, qh = (w.hi[k] >> (8 * slot)) & 255u;
+    const double o = w.o[k], s = w.s15[k];
+    if (!(o + (s + ql * (s / 32768.0)) <= (double)box[k]) || !((double)box[3 + k] <= o + (s + qh * (s / 32768.0))))
+      return false;
+  }
+  return true;
+}
+
+bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* leaves, const float* root_box,
+                 int* nodes3, float* boxes) {
+  const int ni = n - 1;
+  const uint32_t mask = (1u << 30) - 1;
+  for (int x = 0; x < ni + n; x++) nodes3[3 * x] = x == 0 ? -1 : (int)(parent[x] & mask);
+  for (int x = 1; x < ni + n; x++) {
+    const int p = nodes3[3 * x];
+    if (p < 0 || p >= ni) return false;
+    nodes3[3 * p + ((parent[x] >> 31) ? 1 : 2)] = x;
+  }
+  // boxes: the leaves' from their triangles, then unions upwards, the second child to arrive taking its parent's
+  std::vector<char> seen(ni > 0 ? ni : 1, 0);
+  for (int k = 0; k < n; k++) {
+    const LeafTri& t = leaves[k];
+    const float v[3][3] = {{t.v0.x, t.v0.y, t.v0.z}, {t.v1.x, t.v1.y, t.v1.z}, {t.v2.x, t.v2.y, t.v2.z}};
+    int x = ni + k;
+    float* bx = boxes + 6 * (size_t)x;
+    for (int c = 0; c < 3; c++) {
+      bx[c] = std::fmin(v[2][c], std::fmin(v[0][c], v[1][c]));
+      bx[3 + c] = std::fmax(v[2][c], std::fmax(v[0][c], v[1][c]));
+    }
+    while (x != 0 && n > 1) {
+      const int p = nodes3[3 * x];
+      if (seen[p]++ == 0) break;
+      if (seen[p] > 2) return false;
+      const float *l = boxes + 6 * (size_t)nodes3[3 * p + 1], *r = boxes + 6 * (size_t)nodes3[3 * p + 2];
+      float* o = boxes + 6 * (size_t)p;
+      for (int c = 0; c < 3; c++) o[c] = std::fmin(l[c], r[c]), o[3 + c] = std::fmax(l[3 + c], r[3 + c]);
+      x = p;
+    }
+  }
+  if (std::memcmp(boxes, root_box, 6 * sizeof(float)) != 0 && n > 1) return false;
+  // every slot of every wide node names the right node and contains its box (where the traversal looks at boxes)
+  bool filtered = true;
+  for (int c = 0; c < 6; c++) filtered = filtered && std::fabs(root_box[c]) <= kMaxFilterCoord;
+  auto code_of = [&](int x) { return x < ni ? x : ~(x - ni); };
+  for (int i = 0; i < ni; i++)
+    for (int s = 0; s < 4; s++) {
+      const int c = nodes3[3 * i + 1 + (s >> 1)];
+      int x = c;
+      if (c >= ni) {
+        if (s & 1) {
+          if (wn[i].code[s] != kNoChild) return false;
+          continue;
+        }
+      } else {
+        x = nodes3[3 * c + 1 + (s & 1)];
+      }
+      if (wn[i].code[s] != code_of(x) || (filtered && !slot_contains(wn[i], s, boxes + 6 * (size_t)x)))
+        return false;
+    }
+  return true;
+}
 }  // namespace crt
 
 extern "C" {
@@ -227,12 +293,12 @@ static crt_status create_scene(const crt_mesh_desc* d, void* stream, bool borrow
   const int tiles = sort_tiles(n > 0 ? n : 1);
   const size_t nn = n > 0 ? 2 * (size_t)n - 1 : 0;
   const size_t n1 = n > 0 ? (size_t)n : 1;
-  size_t off[13], total = 0;
-  const size_t sizes[13] = {4 * (size_t)n, 4 * (size_t)n, 4 * (size_t)n, 4 * (size_t)n, 4 * 3 * (size_t)kRadix,
+  size_t off[15], total = 0;
+  const size_t sizes[15] = {4 * (size_t)n, 4 * (size_t)n, 4 * (size_t)n, 4 * (size_t)n, 4 * 3 * (size_t)kRadix,
                             4 * 3 * (size_t)tiles * kRadix, 4 * nn, sizeof(uint4) * n1,
                             sizeof(float) * 6 * n1, sizeof(float) * 6 * n1, sizeof(int) * 6 * span_groups(n),
-                            sizeof(LeafTri) * n1, sizeof(WNode) * n1};
-  for (int i = 0; i < 13; i++) off[i] = total, total += align256(sizes[i]);
+                            sizeof(LeafTri) * n1, sizeof(WNode) * n1, 2 * sizeof(float4) * n1, sizeof(int) * n1};
+  for (int i = 0; i < 15; i++) off[i] = total, total += align256(sizes[i]);
   const size_t goff = total;
   total += align256(sizeof(SceneGlobals));
   ALLOC(s->block, total);
@@ -252,6 +318,8 @@ static crt_status create_scene(const crt_mesh_desc* d, void* stream, bool borrow
   b.gbox = reinterpret_cast<int*>(base + off[10]);
   b.leaves = reinterpret_cast<LeafTri*>(base + off[11]);
   b.wnodes = reinterpret_cast<WNode*>(base + off[12]);
+  b.nbox = reinterpret_cast<float4*>(base + off[13]);
+  b.split = reinterpret_cast<int*>(base + off[14]);
   b.g = reinterpret_cast<SceneGlobals*>(base + goff);
   if ((e = cudaMemsetAsync(b.g, 0, sizeof(SceneGlobals), st)) != cudaSuccess) return bail(e, "memset");
   // upload
@@ -369,41 +437,25 @@ crt_status crt_bvh_export(crt_scene* s, float* scene_box, int32_t* codes, uint32
   std::vector<float> box(6);
   for (int k = 0; k < 3; k++) box[k] = ord2f_h(g.bmin[k]), box[3 + k] = ord2f_h(g.bmax[k]);
   std::vector<uint32_t> hk(n), hv(n);
-  std::vector<int> parent(nn);
-  std::vector<WNode> wn(n > 1 ? n : 0);
+  std::vector<uint32_t> parent(nn);
+  std::vector<LeafTri> lf(n);
+  std::vector<WNode> wn(n > 1 ? n - 1 : 0);
   if (n > 0) {
     CRT_CUDA(cudaMemcpy(hk.data(), s->b.keys_b, 4 * (size_t)n, cudaMemcpyDeviceToHost), "download");
     CRT_CUDA(cudaMemcpy(hv.data(), s->b.vals_b, 4 * (size_t)n, cudaMemcpyDeviceToHost), "download");
     CRT_CUDA(cudaMemcpy(parent.data(), s->b.parent, 4 * nn, cudaMemcpyDeviceToHost), "download");
+    CRT_CUDA(cudaMemcpy(lf.data(), s->b.leaves, sizeof(LeafTri) * (size_t)n, cudaMemcpyDeviceToHost), "download");
   }
-  if (n > 1) CRT_CUDA(cudaMemcpy(wn.data(), s->b.wnodes, sizeof(WNode) * (size_t)n, cudaMemcpyDeviceToHost), "download");
+  if (n > 1)
+    CRT_CUDA(cudaMemcpy(wn.data(), s->b.wnodes, sizeof(WNode) * (size_t)(n - 1), cudaMemcpyDeviceToHost), "download");
   std::vector<int> n3(3 * nn);
   std::vector<float> nb(6 * nn);
-  auto ref = [n](int code) { return code >= 0 ? code : (n - 1) + ~code; };
-  for (size_t i = 0; i < nn; i++) n3[3 * i] = (i == 0) ? -1 : (int)((uint32_t)parent[i] & ((1u << 30) - 1));
+  if (n > 0 && !export_tree(n, parent.data(), wn.data(), lf.data(), g.root_box, n3.data(), nb.data()))
+    return fail(CRT_CUDA_ERROR, "inconsistent tree");
   for (int k = 0; k < n; k++) {
     n3[3 * ((n - 1) + k) + 1] = (int)hv[k];
     n3[3 * ((n - 1) + k) + 2] = (int)hv[k];
   }
-  // the children of internal node i sit in the wide node of its parent (the
-  // root's in the virtual node n - 1), slots 2*side(i) and 2*side(i) + 1
-  for (int i = 0; i < n - 1; i++) {
-    const uint32_t w = (uint32_t)parent[i];
-    const int gp = i == 0 ? n - 1 : (int)(w & ((1u << 30) - 1));
-    if (gp < 0 || gp >= n) return fail(CRT_CUDA_ERROR, "inconsistent tree");
-    const int s0 = (i == 0 || (w >> 31)) ? 0 : 2;
-    for (int c = 0; c < 2; c++) {
-      const WSlot& q = wn[gp].s[s0 + c];
-      int code;
-      std::memcpy(&code, &q.lo_code.w, 4);
-      const int r = ref(code);
-      if (code == kNoChild || r < 0 || (size_t)r >= nn) return fail(CRT_CUDA_ERROR, "inconsistent tree");
-      n3[3 * i + 1 + c] = r;
-      const float box[6] = {q.lo_code.x, q.lo_code.y, q.lo_code.z, q.hi.x, q.hi.y, q.hi.z};
-      std::memcpy(&nb[6 * (size_t)r], box, sizeof(box));
-    }
-  }
-  if (nn > 0) std::memcpy(&nb[0], g.root_box, 6 * sizeof(float));
   auto put = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     if (!dst || !bytes) return cudaSuccess;
     return cudaMemcpy(dst, src, bytes, cudaMemcpyDefault);
@@ -656,12 +708,11 @@ crt_status crt_hierarchy(const uint32_t* codes, const uint32_t* ids, int32_t n, 
     return fail(CRT_INVALID_ARG, "crt_hierarchy takes device pointers");
   cudaStream_t st = S(stream);
   const size_t nn = 2 * (size_t)n - 1;
-  const size_t bytes = align256(4 * nn) + sizeof(WNode) * (size_t)n;
+  const size_t bytes = 4 * nn;
   char* scratch = nullptr;
   CRT_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&scratch), bytes, st), "scratch");
   uint32_t* parent = reinterpret_cast<uint32_t*>(scratch);
-  WNode* wnodes = reinterpret_cast<WNode*>(scratch + align256(4 * nn));
-  const cudaError_t e = launch_stage_hierarchy(codes, ids, n, nodes3, parent, wnodes, st);
+  const cudaError_t e = launch_stage_hierarchy(codes, ids, n, nodes3, parent, st);
   CRT_CUDA(cudaFreeAsync(scratch, st), "free");
   CRT_CUDA(e, "hierarchy launch");
   return CRT_OK;

@@ -39,12 +39,14 @@ struct BuildBufs {
   uint32_t* hist = nullptr;    // 3 * kRadix
   uint32_t* status = nullptr;  // 3 * tiles * kRadix
   uint32_t* parent = nullptr;  // 2n - 1: parent index (reference numbering) | left-child and spanning bits
-  uint4* spans = nullptr;      // n: the spanning internal nodes (node, first leaf, last leaf, parent word)
+  uint4* spans = nullptr;      // n: the spanning internal nodes (node, first leaf, last leaf, split)
+  int* split = nullptr;        // n - 1: the last leaf of each internal node's left child
+  float4* nbox = nullptr;      // 2 (n - 1): boxes (lo, hi) of the maximal block-local nodes and of their children
   float* suf = nullptr;        // 6n: box of leaves i..end of i's refit block (at first leaves of block tops;
                                // at a block's first leaf: the block's box)
   float* pre = nullptr;        // 6n: box of leaves start of i's refit block..i (at last leaves of block tops)
   int* gbox = nullptr;         // 6 per group of kSpanGroup refit blocks: the group's box (order-preserving ints)
-  WNode* wnodes = nullptr;     // n (the last one virtual: the root's children)
+  WNode* wnodes = nullptr;     // n - 1
   LeafTri* leaves = nullptr;   // n
   SceneGlobals* g = nullptr;
 };
@@ -72,24 +74,35 @@ struct BatchBufs {
   uint32_t* status = nullptr;  // 4 * tiles * kRadix
   uint32_t* parent = nullptr;  // NI + N
   int* flags = nullptr;        // NI
-  WNode* wnodes = nullptr;     // NI + M (codes local to each mesh; NI + m: mesh m's virtual node)
+  WNode* wnodes = nullptr;     // NI (codes local to each mesh)
+  float4* nbox = nullptr;      // 2 NI: boxes of the maximal block-local nodes, of their children and of the spanning nodes
+  int2* kids = nullptr;        // NI: the children's codes of the maximal block-local and the spanning nodes
   LeafTri* leaves = nullptr;   // N
   SceneGlobals* g = nullptr;   // M
   unsigned* counters = nullptr;  // [0..3] sort tiles, [4] render items, [6] refit hand-offs (8 words)
-  uint2* arrivals = nullptr;     // N: climbs handed from the refit to its spanning-node pass
+  uint4* arrivals = nullptr;     // N: climbs handed from the refit to its spanning-node pass (parent word, mesh, code)
   int* err = nullptr;
 };
 
 int num_sms();
 
+// capi.cu: the reference's nodes (parent, left, right; leaves get their parent
+// only) and exact boxes of a downloaded tree, for the exports: the topology
+// from the parent words (relative to the tree, n >= 1 leaves), the boxes from
+// the leaves' triangles by exact unions.  false when the tree is inconsistent:
+// among the checks, the root box is the device's, and every slot of every wide
+// node names its node and contains that node's box.
+bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* leaves, const float* root_box,
+                 int* nodes3, float* boxes);
+
 // build.cu
 cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st);
 cudaError_t launch_refit(const MeshBufs& m, const BuildBufs& b, cudaStream_t st);
 // Stage-level hierarchy and refit in the reference's HNode layout (scratch:
-// parent 2n - 1 words and wnodes n for the hierarchy; for the refit, flags
-// n - 1 zeroed by the caller).
+// parent 2n - 1 words for the hierarchy; for the refit, flags n - 1 zeroed by
+// the caller).
 cudaError_t launch_stage_hierarchy(const uint32_t* codes, const uint32_t* ids, int n, int* nodes3,
-                                   uint32_t* parent, WNode* wnodes, cudaStream_t st);
+                                   uint32_t* parent, cudaStream_t st);
 cudaError_t launch_stage_refit(const float* V, int nv, const int* vidx, int n, const uint32_t* ids,
                                const int* nodes3, float* boxes, int* flags, int* err, cudaStream_t st);
 // Range checks of device-resident index arrays (kErrIndex in b.g->err).
