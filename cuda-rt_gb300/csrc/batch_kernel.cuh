@@ -458,9 +458,14 @@ __device__ __forceinline__ void ph_render(const BatchView& V, int gmax, int2* ri
     const int W = Ap->W, H = Ap->H;
     const int tiles_x = (W + tw - 1) / tw;
     const int p = lane / G;
-    const int px = (tile % tiles_x) * tw + (p % tw);
-    const int py = (tile / tiles_x) * th + (p / tw);
-    pixel<kRender, SHORT, true>(S, *Ap, px, py, px < W && py < H, G, pred, rb, B, D, ts, glight, ring);
+    const int tx = (tile % tiles_x) * tw, ty = (tile / tiles_x) * th;
+    const int px = tx + (p % tw), py = ty + (p / tw);
+    const bool valid = px < W && py < H;
+    if (beam_misses(S, *Ap, rb, B, tx, tx + tw - 1, ty, ty + th - 1)) {
+      write_miss<kRender>(*Ap, px, py, valid, G, miss_mean(Ap->spp));
+      continue;
+    }
+    pixel<kRender, SHORT, true>(S, *Ap, px, py, valid, G, pred, rb, B, D, ts, glight, ring);
   }
 }
 

@@ -560,78 +560,66 @@ __device__ __forceinline__ int traverse(const DScene& S, const RayC& r, const fl
   const int max_steps = 2 * S.ntri + 64;  // < 2^31 below CRT_MAX_TRIANGLES
   int steps = 0;
   while (true) {
-    // FP32 phase: this lane's next candidate
-    while (run && !pending) {
-      if (node == kPop) {
-        bool next = false;
-        while (stk.sp > 0) {
+    // FP32 phase: this lane's next candidate, a step of every walking lane per
+    // round (the vote also brings the lanes together again)
+    while (__any_sync(0xffffffffu, run && !pending)) {
+      if (run && !pending) {
+        bool got = node != kPop;
+        while (!got && stk.sp > 0) {
           const E e = stk.pop();
-          if (!ANY && entry_bound(e) > pb) continue;
-          node = entry_node(e);
-          next = true;
-          break;
+          if (ANY || !(entry_bound(e) > pb)) node = entry_node(e), got = true;
         }
-        if (!next) {
+        if (!got) {
           run = false;
-          break;
-        }
-      }
-      if (++steps > max_steps || node >= S.ntri - 1 || (node < 0 && (~node & kLeafIndex) >= S.ntri)) {
-        err = true;
-        run = false;
-        break;
-      }
-      if (node >= 0) {
-        if (STATS) ts->nodes++;
-        float L[4], U[4];
-        int c[4];
-        load_slabs<NC>(S.wnodes + node, r, L, U, c);
-        int nhit = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const bool hk = c[k] != kNoChild && (ANY ? L[k] <= U[k] : L[k] <= fminf(U[k], pb));
-          if (!hk) c[k] = kNoChild;
-          if (!ANY && !hk) L[k] = __int_as_float(0x7f800000);
-          nhit += hk ? 1 : 0;
-        }
-        if (!ANY) {  // nearest first; misses (+inf) sort last
-          cswap(L[0], c[0], L[1], c[1]);
-          cswap(L[2], c[2], L[3], c[3]);
-          cswap(L[0], c[0], L[2], c[2]);
-          cswap(L[1], c[1], L[3], c[3]);
-          cswap(L[1], c[1], L[2], c[2]);
-        }
-        if (stk.sp + nhit > kWideStack) {
+        } else if (++steps > max_steps || node >= S.ntri - 1 || (node < 0 && (~node & kLeafIndex) >= S.ntri) ||
+                   stk.sp > kWideStack - 4) {  // only a corrupt tree gets here
           err = true;
           run = false;
-          break;
-        }
-        // take the first hit slot now, stack the others so they pop in order
-        int next = kPop;
-        float tnext = 0.f;
+        } else if (node >= 0) {
+          if (STATS) ts->nodes++;
+          float L[4], U[4];
+          int c[4];
+          load_slabs<NC>(S.wnodes + node, r, L, U, c);
+          node = kPop;
+          if (ANY) {
+            // the first hit slot is next, the others are stacked so they pop in order
 #pragma unroll
-        for (int k = 3; k >= 0; k--) {
-          if (c[k] != kNoChild) {
-            if (next != kPop) stk.push(stack_entry(next, tnext, (E*)nullptr));
-            next = c[k];
-            tnext = L[k];
+            for (int k = 3; k >= 0; k--) {
+              if (L[k] <= U[k] && c[k] != kNoChild) {
+                if (node != kPop) stk.push(stack_entry(node, 0.f, (E*)nullptr));
+                node = c[k];
+              }
+            }
+          } else {
+            // nearest first; misses (+inf) sort last
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              if (!(L[k] <= fminf(U[k], pb) && c[k] != kNoChild)) c[k] = kNoChild, L[k] = __int_as_float(0x7f800000);
+            cswap(L[0], c[0], L[1], c[1]);
+            cswap(L[2], c[2], L[3], c[3]);
+            cswap(L[0], c[0], L[2], c[2]);
+            cswap(L[1], c[1], L[3], c[3]);
+            cswap(L[1], c[1], L[2], c[2]);
+#pragma unroll
+            for (int k = 3; k >= 1; k--)
+              if (c[k] != kNoChild) stk.push(stack_entry(c[k], L[k], (E*)nullptr));
+            node = c[0];
           }
+        } else {
+          if (STATS) ts->tris++;
+          const float4* lp = reinterpret_cast<const float4*>(S.leaves + (~node & kLeafIndex));
+          const float4 a = ld_node<NC>(lp), b = ld_node<NC>(lp + 1), c = ld_node<NC>(lp + 2);
+          if (!tri_reject_sure(r, a, b, c)) {
+            cand = node, pending = true;
+            // the leaf's box (as the refit computes it from the same vertices)
+            // is tested here rather than when the leaf is pushed: one copy of
+            // the test in the walk's code, and none for leaves never reached
+            if (!box_sure(r, fminf(c.x, fminf(a.x, b.x)), fmaxf(c.x, fmaxf(a.x, b.x)), fminf(c.y, fminf(a.y, b.y)),
+                          fmaxf(c.y, fmaxf(a.y, b.y)), fminf(c.z, fminf(a.z, b.z)), fmaxf(c.z, fmaxf(a.z, b.z))))
+              cand = ~(~cand | kLeafBoxDue);
+          }
+          node = kPop;
         }
-        node = next;
-      } else {
-        if (STATS) ts->tris++;
-        const float4* lp = reinterpret_cast<const float4*>(S.leaves + (~node & kLeafIndex));
-        const float4 a = ld_node<NC>(lp), b = ld_node<NC>(lp + 1), c = ld_node<NC>(lp + 2);
-        if (!tri_reject_sure(r, a, b, c)) {
-          cand = node, pending = true;
-          // the leaf's box (as the refit computes it from the same vertices)
-          // is tested here rather than when the leaf is pushed: one copy of
-          // the test in the walk's code, and none for leaves never reached
-          if (!box_sure(r, fminf(c.x, fminf(a.x, b.x)), fmaxf(c.x, fmaxf(a.x, b.x)), fminf(c.y, fminf(a.y, b.y)),
-                        fmaxf(c.y, fmaxf(a.y, b.y)), fminf(c.z, fminf(a.z, b.z)), fmaxf(c.z, fmaxf(a.z, b.z))))
-            cand = ~(~cand | kLeafBoxDue);
-        }
-        node = kPop;
       }
     }
     // double phase: the lanes holding a candidate, together

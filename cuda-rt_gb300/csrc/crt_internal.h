@@ -173,6 +173,7 @@ struct RenderArgs {
 };
 cudaError_t launch_render(const DScene& S, const RenderArgs& a, cudaStream_t st);
 
+
 // The tile rectangles for a tiles_x x tiles_y grid of tiles: with split and a
 // large enough image about num_sms() of them, near square, else one; their
 // counters and bound zeroed on st.

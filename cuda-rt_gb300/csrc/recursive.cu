@@ -25,7 +25,7 @@
 // bit.  The traversals are warp-synchronous: each step of the loop traces
 // the next ray of every lane that has one, then the shadow rays of the lanes
 // whose ray hit.
-#include "crt_internal.h"
+#include "pixel.cuh"
 
 namespace crt {
 
@@ -156,9 +156,14 @@ __global__ void __launch_bounds__(128) k_pixels_rec(DScene S, RenderArgs A, cons
     tile = __shfl_sync(full, tile, 0);
     if (tile < 0) break;
     const int pp = lane / G;  // this lane's pixel in the tile
-    const int px = (tile % tiles_x) * tw + (pp % tw);
-    const int py = A.row0 + (tile / tiles_x) * th + (pp / tw);
+    const int tx = (tile % tiles_x) * tw, ty = A.row0 + (tile / tiles_x) * th;
+    const int px = tx + (pp % tw), py = ty + (pp / tw);
     const bool valid = px < A.W && py < A.row1;
+    if (!A.rays && beam_misses(S, A, rb, B, tx, tx + tw - 1, ty, ty + th - 1)) {
+      write_miss<kRender>(A, px, py, valid, G, miss_mean(A.spp));
+      if (valid && g == 0) nrays += (unsigned)A.spp;
+      continue;
+    }
     const int idx = (A.H - py - 1) * A.W + px;
     uint32_t wst =
         wang_hash((uint32_t)(((py / 16) * gx + px / 16) * 256 + (py % 16) * 16 + (px % 16)) ^ A.seed_mix);

@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(128, 9) k_pixels(DScene S, RenderArgs A) {
   const int tiles_y = (A.row1 - A.row0 + th - 1) / th;
   const int p = lane / G;  // this lane's pixel in the tile
   unsigned pred = 0xffffffffu;
+  const bool cull = MODE == kAdjoint || !A.rays;  // (requested rays have to be made)
+  double miss = 0.0;  // a missing pixel's mean, once this warp has met one
   int region = home_region(A.regions_x, A.regions_y);
   bool home = true;
   while (true) {
@@ -84,9 +86,15 @@ __global__ void __launch_bounds__(128, 9) k_pixels(DScene S, RenderArgs A) {
     if (lane == 0) tile = claim_tile(A.counter, tiles_x, tiles_y, A.regions_x, A.regions_y, region, home);
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if (tile < 0) break;
-    const int px = (tile % tiles_x) * tw + (p % tw);
-    const int py = A.row0 + (tile / tiles_x) * th + (p / tw);
-    pixel<MODE, kPixelsShort>(S, A, px, py, px < A.W && py < A.row1, G, pred, rb, B, D, ts, glight, ring);
+    const int tx = (tile % tiles_x) * tw, ty = A.row0 + (tile / tiles_x) * th;
+    const int px = tx + (p % tw), py = ty + (p / tw);
+    const bool valid = px < A.W && py < A.row1;
+    if (cull && beam_misses(S, A, rb, B, tx, tx + tw - 1, ty, ty + th - 1)) {
+      if (miss == 0.0) miss = miss_mean(A.spp);
+      write_miss<MODE>(A, px, py, valid, G, miss);
+      continue;
+    }
+    pixel<MODE, kPixelsShort>(S, A, px, py, valid, G, pred, rb, B, D, ts, glight, ring);
   }
   flush_stats<MODE>(A, ts, glight);
 }
