@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -76,6 +77,64 @@ DScene dscene(const crt_scene* s) {
   return d;
 }
 
+// Per-call scratch and staging memory comes from a pool of the library's own,
+// one per device, that keeps up to kScratchKept bytes between calls.  (The
+// device's default pool keeps nothing: every call that allocates and then
+// synchronises maps its memory anew.)  Allocation stays stream-ordered, so
+// calls on several streams and threads never share a block.  Destroying a
+// scene gives the kept memory back.  While a stream is captured, on another
+// device's stream, or when the pool cannot serve, the default pool is used.
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kScratchKept = (uint64_t)256 << 20;
+struct ScratchPool {
+  unsigned long long ctx_id = 0;  // the CUDA context the pool was made in
+  cudaMemPool_t pool = nullptr;
+};
+std::mutex g_pool_mu;
+ScratchPool g_pool[kMaxDevices];
+
+// The current context's pool, made on first use (make), or NULL.
+cudaMemPool_t scratch_pool(bool make) {
+  int dev = 0;
+  unsigned long long id = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices || !current_context_id(&id)) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ScratchPool& p = g_pool[dev];
+  if (p.pool && p.ctx_id == id) return p.pool;
+  p.pool = nullptr;
+  if (!make) return nullptr;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  uint64_t kept = kScratchKept;
+  if (cudaMemPoolCreate(&p.pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) {
+    cudaGetLastError();
+    p.pool = nullptr;
+  }
+  p.ctx_id = id;
+  return p.pool;
+}
+
+cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  int dev = 0, sdev = 0;
+  const bool plain = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+                     (st && (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetDevice(st, &sdev) != cudaSuccess ||
+                             dev != sdev));
+  if (!plain)
+    if (cudaMemPool_t p = scratch_pool(true)) {
+      if (cudaMallocFromPoolAsync(out, bytes, p, st) == cudaSuccess) return cudaSuccess;
+      cudaGetLastError();
+    }
+  return cudaMallocAsync(out, bytes, st);
+}
+
+void scratch_trim() {
+  if (cudaMemPool_t p = scratch_pool(false)) cudaMemPoolTrimTo(p, 0);
+}
+
 // A device view of a caller buffer: the buffer itself when it is device
 // memory, else a stream-ordered temporary that is copied in and/or out.
 struct DevView {
@@ -92,7 +151,7 @@ struct DevView {
       return cudaSuccess;
     }
     temp = true;
-    cudaError_t e = cudaMallocAsync(&dev, n, st);
+    cudaError_t e = scratch_alloc(&dev, n, st);
     if (e != cudaSuccess) return e;
     if (copy_in) return cudaMemcpyAsync(dev, p, n, cudaMemcpyDefault, st);
     return cudaSuccess;
@@ -379,6 +438,7 @@ crt_status crt_scene_destroy(crt_scene* s) {
   cudaDeviceSynchronize();
   free_scene(s);
   delete s;
+  scratch_trim();
   return CRT_OK;
 }
 
@@ -658,7 +718,7 @@ crt_status crt_adjoint_lambert(crt_scene* s, const crt_camera* cam, const crt_li
   // gradient outputs: always through device scratch (they are accumulated atomically)
   const size_t nv3 = 3 * (size_t)s->m.nv, nk3 = 3 * (size_t)s->m.nmat;
   double* acc = nullptr;
-  CRT_CUDA(cudaMallocAsync(&acc, sizeof(double) * (nv3 + 3 + nk3), st), "scratch");
+  CRT_CUDA(scratch_alloc(reinterpret_cast<void**>(&acc), sizeof(double) * (nv3 + 3 + nk3), st), "scratch");
   CRT_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * (nv3 + 3 + nk3), st), "memset");
   a.grad_rgb = static_cast<const double*>(vg.dev);
   a.grad_depth = static_cast<const double*>(vgd.dev);
@@ -688,7 +748,7 @@ crt_status crt_morton(const float* verts, int32_t num_vertices, const int32_t* v
     return fail(CRT_INVALID_ARG, "crt_morton takes device pointers");
   cudaStream_t st = S(stream);
   int* scratch = nullptr;  // error bit
-  CRT_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&scratch), sizeof(int), st), "scratch");
+  CRT_CUDA(scratch_alloc(reinterpret_cast<void**>(&scratch), sizeof(int), st), "scratch");
   CRT_CUDA(cudaMemsetAsync(scratch, 0, sizeof(int), st), "memset");
   const cudaError_t e =
       launch_morton(verts, num_vertices, vidx, n, box6, reinterpret_cast<uint32_t*>(codes), scratch, st);
@@ -710,7 +770,7 @@ crt_status crt_hierarchy(const uint32_t* codes, const uint32_t* ids, int32_t n, 
   const size_t nn = 2 * (size_t)n - 1;
   const size_t bytes = 4 * nn;
   char* scratch = nullptr;
-  CRT_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&scratch), bytes, st), "scratch");
+  CRT_CUDA(scratch_alloc(reinterpret_cast<void**>(&scratch), bytes, st), "scratch");
   uint32_t* parent = reinterpret_cast<uint32_t*>(scratch);
   const cudaError_t e = launch_stage_hierarchy(codes, ids, n, nodes3, parent, st);
   CRT_CUDA(cudaFreeAsync(scratch, st), "free");
@@ -729,7 +789,7 @@ crt_status crt_refit(const float* vertices, int32_t num_vertices, const int32_t*
     return fail(CRT_INVALID_ARG, "crt_refit takes device pointers");
   cudaStream_t st = S(stream);
   int* scratch = nullptr;  // [0] error bits, [1..n-1] arrival flags
-  CRT_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&scratch), 4 * (size_t)n, st), "scratch");
+  CRT_CUDA(scratch_alloc(reinterpret_cast<void**>(&scratch), 4 * (size_t)n, st), "scratch");
   CRT_CUDA(cudaMemsetAsync(scratch, 0, 4 * (size_t)n, st), "memset");
   const cudaError_t e = launch_stage_refit(vertices, num_vertices, vertex_indices, n, ids, nodes3, node_boxes,
                                            scratch + 1, scratch, st);
@@ -751,7 +811,7 @@ crt_status crt_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ko
   cudaStream_t st = S(stream);
   const size_t bytes = sort_scratch_bytes(n, key_bits) + 256;
   void* scratch = nullptr;
-  CRT_CUDA(cudaMallocAsync(&scratch, bytes, st), "scratch");
+  CRT_CUDA(scratch_alloc(&scratch, bytes, st), "scratch");
   int* err = reinterpret_cast<int*>(static_cast<char*>(scratch) + bytes - 256);
   cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
   if (e == cudaSuccess) e = launch_sort_pairs(kin, vin, kout, vout, n, key_bits, scratch, err, st);

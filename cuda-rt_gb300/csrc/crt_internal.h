@@ -86,6 +86,10 @@ struct BatchBufs {
 
 int num_sms();
 
+// sort_noalloc.cu: the id of the current CUDA context, unique for the life of
+// the process (a context that cudaDeviceReset destroyed never comes back).
+bool current_context_id(unsigned long long* id);
+
 // capi.cu: the reference's nodes (parent, left, right; leaves get their parent
 // only) and exact boxes of a downloaded tree, for the exports: the topology
 // from the parent words (relative to the tree, n >= 1 leaves), the boxes from

@@ -35,6 +35,34 @@ void set_last_error(const char* msg);
 }
 
 namespace {
+// cuCtxGetCurrent and cuCtxGetId through the runtime's driver entry points
+// (no link-time dependence on libcuda): a context's id is unique for the
+// life of the process, so an address looked up in a context that
+// cudaDeviceReset has since destroyed is never reused.
+typedef int (*CtxGetCurrentFn)(void** ctx);
+typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
+void* driver_fn(const char* name) {
+  void* f = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return f;
+}
+}  // namespace
+
+namespace crt {
+bool current_context_id(unsigned long long* id) {
+  static CtxGetCurrentFn get_current = reinterpret_cast<CtxGetCurrentFn>(driver_fn("cuCtxGetCurrent"));
+  static CtxGetIdFn get_id = reinterpret_cast<CtxGetIdFn>(driver_fn("cuCtxGetId"));
+  void* ctx = nullptr;
+  return get_current && get_id && get_current(&ctx) == 0 && ctx && get_id(ctx, id) == 0;
+}
+}  // namespace crt
+
+namespace {
 
 constexpr size_t kMaxPairs = CRT_SORT_NOALLOC_MAX_PAIRS;
 constexpr size_t kMaxPasses = 4;  // 32-bit keys, 10-bit digits
@@ -54,29 +82,6 @@ struct ScratchAddr {
 };
 ScratchAddr g_scratch_addr[kMaxDevices];
 
-// cuCtxGetCurrent and cuCtxGetId through the runtime's driver entry points
-// (no link-time dependence on libcuda): a context's id is unique for the
-// life of the process, so an address looked up in a context that
-// cudaDeviceReset has since destroyed is never reused.
-typedef int (*CtxGetCurrentFn)(void** ctx);
-typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
-void* driver_fn(const char* name) {
-  void* f = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-      q != cudaDriverEntryPointSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return f;
-}
-bool current_context_id(unsigned long long* id) {
-  static CtxGetCurrentFn get_current = reinterpret_cast<CtxGetCurrentFn>(driver_fn("cuCtxGetCurrent"));
-  static CtxGetIdFn get_id = reinterpret_cast<CtxGetIdFn>(driver_fn("cuCtxGetId"));
-  void* ctx = nullptr;
-  return get_current && get_id && get_current(&ctx) == 0 && ctx && get_id(ctx, id) == 0;
-}
-
 // The device address of g_sort_scratch in the current context, looked up
 // once per context with its device current.
 cudaError_t scratch_on_current_device(void** out) {
@@ -87,7 +92,7 @@ cudaError_t scratch_on_current_device(void** out) {
   e = cudaSetDevice(dev);  // initialises the device's primary context and makes it current
   if (e != cudaSuccess) return e;
   unsigned long long id = 0;
-  if (!current_context_id(&id)) return cudaErrorInitializationError;
+  if (!crt::current_context_id(&id)) return cudaErrorInitializationError;
   std::lock_guard<std::mutex> lk(g_mu);
   ScratchAddr& c = g_scratch_addr[dev];
   if (!c.addr || c.ctx_id != id) {
