@@ -72,7 +72,7 @@ struct BatchLaunch {
   BatchView v;
   int gmax;         // the most lanes a pixel may take (lanes per pixel option)
   int sort_tiles;   // tiles of one sort pass
-  unsigned* bar;    // grid barrier: [0] arrivals, [1] generation (both 0 at launch)
+  unsigned* bar;    // grid barrier: arrivals (0 at launch)
   int first, last;  // the phases to run
 };
 
@@ -494,8 +494,9 @@ __global__ void __launch_bounds__(TH, 1024 / TH) k_batch(const BatchBufs b, cons
   RefitSmem& refit_sm = *reinterpret_cast<RefitSmem*>(smem);
   uint32_t* morton_sm = reinterpret_cast<uint32_t*>(smem);
   int2* ring = SHORT > 0 ? reinterpret_cast<int2*>(smem) + threadIdx.x : nullptr;
+  unsigned passed = 0;  // grid barriers
   for (int ph = first; ph <= last; ph++) {
-    if (ph > first && !grid_barrier(bar, gridDim.x, b.err)) return;
+    if (ph > first && !grid_barrier(bar, gridDim.x, passed, b.err)) return;
     switch (ph) {
       case kPhInit:
         ph_init(b);

@@ -192,22 +192,22 @@ __global__ void k_zero_u32(uint32_t* p, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = 0;
 }
 
-// All passes of the build's stable LSD sort in one cooperative launch, one
-// 8192-key tile per block (so at most as many tiles as blocks that fit on the
-// GPU at once; launch_build falls back to k_onesweep passes beyond that).
-// Within a pass every block ranks its tile as k_onesweep does, publishes its
-// per-digit counts, and after a grid-wide barrier sums the counts of all
-// tiles, keeping apart those of the tiles before it (up to a few hundred
-// independent loads per thread instead of a chain of look-back round trips):
-// the digit totals give each digit's start, so no histogram pass precedes the
-// sort.  Then it scatters; a second barrier ends the pass.  Pass p reads keys_a (p even) or keys_b and writes the other
-// array (values likewise; pass 0 takes values 0..n-1).  Barrier words:
-// bar[0..1], zero at launch; a barrier that waits too long sets kErrTimeout
-// in *err and the kernel stops.
+// All passes of a stable LSD sort in one cooperative launch, one tile of
+// 1024 * IT keys per block (so at most as many tiles as blocks that fit on the
+// GPU at once; the k_onesweep passes take over beyond that).  Within a pass
+// every block ranks its tile as k_onesweep does and publishes its per-digit
+// counts; after a grid-wide barrier it sums all tiles' counts itself, keeping
+// apart those of the tiles before it (independent loads; no histogram pass
+// precedes the sort).  (Scanning each digit's column over the tiles once, with
+// one more barrier, reads ntiles rows instead of ntiles^2 but was 4 us a pass
+// slower at 140 tiles.)  Then it scatters; a barrier ends the pass.  Pass 0 reads kin and vin (NULL: values 0..n-1); pass p
+// writes X (p even) or Y and the next one reads it; kin may be Y.  counts
+// holds ntiles rows.  Barrier word: bar[0], zero at launch; a
+// barrier that waits too long sets kErrTimeout in *err and the kernel stops.
 template <int TH, int IT>
-__global__ void __launch_bounds__(TH, 1) k_sort_coop(uint32_t* keys_a, uint32_t* keys_b, uint32_t* vals_a,
-                                                     uint32_t* vals_b, int n, int passes, uint32_t* counts,
-                                                     unsigned* bar, int* err) {
+__global__ void __launch_bounds__(TH, 1) k_sort_coop(const uint32_t* kin0, const uint32_t* vin0, uint32_t* kx,
+                                                     uint32_t* vx, uint32_t* ky, uint32_t* vy, int n, int passes,
+                                                     uint32_t* counts, unsigned* bar, int* err) {
   constexpr int W = TH / 32;
   constexpr int TILE = TH * IT;
   constexpr int DPT = kRadix / TH;
@@ -218,11 +218,12 @@ __global__ void __launch_bounds__(TH, 1) k_sort_coop(uint32_t* keys_a, uint32_t*
   const uint32_t mask = kRadix - 1;
   unsigned short* wh = reinterpret_cast<unsigned short*>(sm.whist[warp]);
   const uint32_t lt = lanemask_lt();
+  unsigned passed = 0;  // grid barriers
   for (int p = 0; p < passes; p++) {
-    const uint32_t* kin = (p & 1) ? keys_b : keys_a;
-    const uint32_t* vin = p == 0 ? nullptr : ((p & 1) ? vals_b : vals_a);
-    uint32_t* kout = (p & 1) ? keys_a : keys_b;
-    uint32_t* vout = (p & 1) ? vals_a : vals_b;
+    const uint32_t* kin = p == 0 ? kin0 : ((p & 1) ? kx : ky);
+    const uint32_t* vin = p == 0 ? vin0 : ((p & 1) ? vx : vy);
+    uint32_t* kout = (p & 1) ? ky : kx;
+    uint32_t* vout = (p & 1) ? vy : vx;
     const int shift = p * kRadixBits;
     // each warp clears its own counters (no other warp reads them before the
     // block's next __syncthreads)
@@ -270,17 +271,14 @@ __global__ void __launch_bounds__(TH, 1) k_sort_coop(uint32_t* keys_a, uint32_t*
       cnt[j] = c;
       csum += c;
     }
-    uint32_t* mine = counts + ((size_t)p * ntiles + tile) * kRadix;
+    uint32_t* mine = counts + (size_t)tile * kRadix;
 #pragma unroll
-    for (int j = 0; j < DPT; j++) mine[DPT * tid + j] = cnt[j];
-    if (!grid_barrier(bar, ntiles, err)) return;
-    // each digit's count over the tiles before this one, and over all tiles
-    // (every block reads every tile's counts: no longer than the last
-    // block's prefix alone, which the pass waits for anyway)
+    for (int j = 0; j < DPT; j++) __stcg(mine + DPT * tid + j, cnt[j]);
+    if (!grid_barrier(bar, ntiles, passed, err)) return;
     uint32_t pre[DPT], tot[DPT], gsum = 0;
 #pragma unroll
     for (int j = 0; j < DPT; j++) {
-      const uint32_t* col = counts + (size_t)p * ntiles * kRadix + DPT * tid + j;
+      const uint32_t* col = counts + DPT * tid + j;
       // 32 loads in flight per round (each round waits one L2 round trip)
       constexpr int U = 32;
       uint32_t acc = 0u, all = 0u;
@@ -331,7 +329,7 @@ __global__ void __launch_bounds__(TH, 1) k_sort_coop(uint32_t* keys_a, uint32_t*
       kout[pos] = k;
       vout[pos] = sm.vals[i];
     }
-    if (p + 1 < passes && !grid_barrier(bar, ntiles, err)) return;
+    if (p + 1 < passes && !grid_barrier(bar, ntiles, passed, err)) return;
   }
 }
 
@@ -800,20 +798,55 @@ static void refit(const MeshBufs& m, const BuildBufs& b, cudaStream_t st) {
              (const float*)b.pre, (const int*)b.gbox, n, b.g);
 }
 
-// Whether the build's sort runs as one cooperative launch (k_sort_coop): its
-// 8192-key tiles must all be resident at once.
-static bool coop_sort_fits(int n) {
-  static int capacity = -1;
+// The cooperative sort's shape (items per thread) for n keys, -1 when it does
+// not take them: the fewest items that leave no more tiles than SMs, so that as
+// many SMs as possible rank keys.  (With 8 items whatever n, 19,220 keys were
+// three tiles and took 57 us; a 100,000-triangle build falls from 109 to 92 us,
+// 40,000 from 117 to 78, 19,220 from 84 to 61; at 1,003,520 7 items instead of
+// 8 and the shorter barrier make it 211.5 us from 216.5.)  The build takes it
+// from kCoopBuildMin keys on: below, three look-back passes launched as
+// programmatic dependents cost less than the cooperative launch (2000
+// triangles 43 against 54 us, 16,000 58 against 61).  The standalone sort,
+// which would also need a histogram pass, takes it from 1025 keys on (3000
+// 16-bit keys 55 against 64 us, 20,000 32-bit ones 73 against 78, 1,000,003
+// 131 against 137).
+constexpr int kCoopBuildMin = 2 * kSortTileL, kCoopSortMin = kSortThreadsL + 1;
+using CoopSort = void (*)(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, int, int,
+                          uint32_t*, unsigned*, int*);
+constexpr int kCoopItems[] = {1, 2, 4, 7, 8};
+constexpr CoopSort kCoopSort[] = {k_sort_coop<kSortThreadsL, 1>, k_sort_coop<kSortThreadsL, 2>,
+                                  k_sort_coop<kSortThreadsL, 4>, k_sort_coop<kSortThreadsL, 7>,
+                                  k_sort_coop<kSortThreadsL, 8>};
+constexpr int kCoopShapes = sizeof(kCoopItems) / sizeof(kCoopItems[0]);
+static int coop_shape(int n, int least) {
+  static int capacity = -1;  // one block per SM at least, or none
   if (capacity < 0) {
     int bps = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_sort_coop<kSortThreadsL, kSortItems>, kSortThreadsL, 0) !=
-        cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kCoopSort[kCoopShapes - 1], kSortThreadsL, 0) != cudaSuccess) {
       cudaGetLastError();
       bps = 0;
     }
-    capacity = bps * num_sms();
+    capacity = bps > 0 ? num_sms() : 0;
   }
-  return n >= 2 * kSortTileL && (n + kSortTileL - 1) / kSortTileL <= capacity;
+  if (n < least) return -1;
+  for (int i = 0; i < kCoopShapes; i++)
+    if (((int64_t)n + kSortThreadsL * kCoopItems[i] - 1) / (kSortThreadsL * kCoopItems[i]) <= capacity) return i;
+  return -1;
+}
+static cudaError_t launch_coop_sort(int shape, const uint32_t* kin, const uint32_t* vin, uint32_t* kx, uint32_t* vx,
+                                    uint32_t* ky, uint32_t* vy, int n, int passes, uint32_t* counts,
+                                    unsigned* bar, int* err, cudaStream_t st) {
+  const int tile = kSortThreadsL * kCoopItems[shape];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n + tile - 1) / tile));
+  cfg.blockDim = dim3(kSortThreadsL);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kCoopSort[shape], kin, vin, kx, vx, ky, vy, n, passes, counts, bar, err);
 }
 
 cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st) {
@@ -821,7 +854,8 @@ cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st)
   if (n <= 0) return cudaSuccess;
   const int passes = 3;
   const int tiles = sort_tiles(n);
-  const bool coop = coop_sort_fits(n);
+  const int shape = coop_shape(n, kCoopBuildMin);
+  const bool coop = shape >= 0;
   k_build_init<<<1, 1024, 0, st>>>(b.g, b.hist, passes * kRadix, b.gbox, (int)span_groups(n));
   const int sms = num_sms();
   const int gb = min((n + 255) / 256, sms * 8);
@@ -836,18 +870,10 @@ cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st)
              (const SceneGlobals*)b.g, b.keys_a, b.hist, passes, b.status, passes * tiles * kRadix);
   // pass 0: keys_a -> keys_b (values 0..n-1), pass 1: b -> a, pass 2: a -> b
   if (coop) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((n + kSortTileL - 1) / kSortTileL));
-    cfg.blockDim = dim3(kSortThreadsL);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    // barrier words: tile_counter[0..1], zeroed by k_build_init
-    cudaLaunchKernelEx(&cfg, k_sort_coop<kSortThreadsL, kSortItems>, b.keys_a, b.keys_b, b.vals_a, b.vals_b, n,
-                       passes, b.status, &b.g->tile_counter[0], &b.g->err);
+    // (counts: ntiles rows of the look-back status; barrier word:
+    // tile_counter[0], zeroed by k_build_init)
+    launch_coop_sort(shape, b.keys_a, nullptr, b.keys_b, b.vals_b, b.keys_a, b.vals_a, n, passes, b.status,
+                     &b.g->tile_counter[0], &b.g->err, st);
   } else {
     const uint32_t* kin = b.keys_a;
     const uint32_t* vin = nullptr;
@@ -1051,6 +1077,15 @@ cudaError_t launch_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t
   uint32_t* hist = w + 2 * (size_t)n;
   uint32_t* status = hist + passes * kRadix;
   unsigned* counters = status + (size_t)passes * tiles * kRadix;
+  // (one pass leaves room for half the rows that 1024-key tiles need)
+  const int shape = passes >= 2 ? coop_shape(n, kCoopSortMin) : -1;
+  if (shape >= 0) {
+    const cudaError_t e = cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    uint32_t *kx = (passes & 1) ? kout : tk, *vx = (passes & 1) ? vout : tv;
+    uint32_t *ky = (passes & 1) ? tk : kout, *vy = (passes & 1) ? tv : vout;
+    return launch_coop_sort(shape, kin, vin, kx, vx, ky, vy, n, passes, status, counters, err, st);
+  }
   k_zero_u32<<<1, 256, 0, st>>>(hist, passes * kRadix);
   k_zero_u32<<<1, 32, 0, st>>>(counters, 4);
   const int gm = min((n + 511) / 512, num_sms() * 2);

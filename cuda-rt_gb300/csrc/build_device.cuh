@@ -232,15 +232,12 @@ __device__ __forceinline__ void block_excl_scan2(uint32_t a, uint32_t b, unsigne
 
 constexpr uint32_t kFlagAgg = 1u << 30, kFlagInc = 2u << 30, kValMask = (1u << 30) - 1;
 
-constexpr int kBarrierSpinLimit = 1 << 22;  // bounded barrier wait (x ~100 ns)
+constexpr int kBarrierSpinLimit = 1 << 22;  // bounded barrier wait (polls of some 0.5 us)
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ unsigned atom_add_acq_rel_u32(unsigned* p, unsigned v) {
   unsigned old;
@@ -249,28 +246,29 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_u32(unsigned* p, unsigned v
 }
 
 // Grid-wide barrier over all `nblocks` blocks: every write made before it by
-// any thread of the grid is visible to every thread after it.  Returns false
+// any thread of the grid is visible to every thread after it.  bar[0] counts
+// arrivals from 0 at launch; `passed`, the caller's count of barriers so far,
+// gives the arrivals to wait for, so a barrier is one add and polls of one
+// word.  (A generation word, read before the add and released after it, and a
+// sleep between polls made a barrier of two blocks take 15 us.)  Returns false
 // (and sets kErrTimeout) when the wait gave up; the caller then stops.
-__device__ __noinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, int* err) {
+__device__ __noinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, unsigned& passed, int* err) {
   __shared__ int s_ok;
   __syncthreads();
+  passed++;
   if (threadIdx.x == 0) {
     int ok = 1;
     __threadfence();
-    const unsigned gen = ld_acquire_u32(bar + 1);
-    if (atom_add_acq_rel_u32(bar, 1u) == nblocks - 1) {
-      atomicExch(bar, 0u);
-      st_release_u32(bar + 1, gen + 1);
-    } else {
+    const unsigned target = passed * nblocks;
+    if (atom_add_acq_rel_u32(bar, 1u) + 1u != target) {
       int spins = 0;
-      while (ld_acquire_u32(bar + 1) == gen) {
+      while (ld_acquire_u32(bar) < target) {
         if (++spins > kBarrierSpinLimit ||
             ((spins & 1023) == 0 && (ld_relaxed(reinterpret_cast<const uint32_t*>(err)) & kErrTimeout))) {
           atomicOr(err, kErrTimeout);
           ok = 0;
           break;
         }
-        __nanosleep(64);
       }
     }
     __threadfence();
