@@ -253,7 +253,7 @@ __device__ __forceinline__ void pixel(const DScene& S, const RenderArgs& A, int 
           ray_setup(rc, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, B, D);
         }
         HitRec ht;
-        const int r = traverse<false, MODE == kRenderStats, SHORT, NC>(S, rc, rb, ht, !done, &ts, ring);
+        const int r = traverse<false, MODE == kRenderStats, SHORT, NC, true>(S, rc, rb, ht, !done, &ts, ring);
         if (!done) h = ht, res = r;
         hits = __ballot_sync(full, act && res > 0);
         // a lane is settled when every earlier sample of its group was guessed right
@@ -290,7 +290,10 @@ __device__ __forceinline__ void pixel(const DScene& S, const RenderArgs& A, int 
       wst = __shfl_sync(full, st, base + G - 1);
       // Light::shadowAttenuation: any-hit from q towards the light
       HitRec s;
-      const int sres = traverse<true, MODE == kRenderStats, SHORT, NC>(S, sr, rb, s, hit, &ts, ring);
+      sr.oself = fabsf((float)A.aperture);  // (at least the lens radius, which bounds the primary ray's origin)
+      const int sres =
+          traverse<true, MODE == kRenderStats, SHORT, NC, true>(S, sr, rb, s, hit, &ts, ring, (float)dist,
+                                                                hit ? h.id : -1);
       if (sres < 0) atomicOr(&S.g->err, kErrStack);
       D3 N;
       double sN = 0.0, fall = 0.0, datt = 0.0;
@@ -321,7 +324,7 @@ __device__ __forceinline__ void pixel(const DScene& S, const RenderArgs& A, int 
         int omid = -1;
         bool otrans = false;
         DMat om;
-        if (sres > 0 && s.t < dist && !(s.t < kRayEps)) {  // dist = norm(lpos - q), Light.cu:14-16
+        if (sres > 0) {
           sh = 1;
           shid = s.id;
           omid = __ldg(S.matid + s.id);

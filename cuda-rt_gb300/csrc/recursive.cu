@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(128) k_pixels_rec(DScene S, RenderArgs A, cons
             ray_setup(sr, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, B, D);
           }
           HitRec sh;
-          const int sres = traverse<true>(S, sr, rb, sh, hit);
+          const int sres = traverse<true>(S, sr, rb, sh, hit, nullptr, nullptr, (float)dist);
           if (sres < 0) atomicOr(&S.g->err, kErrStack);
           if (!busy) continue;
           // Material::shade (kernels/material.cu:6-40), as the plain pixel kernel
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(128) k_pixels_rec(DScene S, RenderArgs A, cons
             fall = fabs(fall) < kRayEps ? 1.0 : 1.0 / fall;
             const double datt = fmin(1.0, fall);
             D3 satt = d3(1, 1, 1);
-            if (sres > 0 && sh.t < dist && !(sh.t < kRayEps)) {
+            if (sres > 0) {
               const DMat& om = S.mats[__ldg(S.matid + sh.id)];
               const bool otrans = om.kt[0] == 0 && om.kt[1] == 0 && om.kt[2] == 0;  // Trans() = isZero(kt)
               satt = otrans ? d3(om.kd[0] * (1 - om.kt[0]), om.kd[1] * (1 - om.kt[1]), om.kd[2] * (1 - om.kt[2]))

@@ -1,0 +1,62 @@
+"""The pixel kernels' hits that FP32 settles (certain closest hits, a shadow ray's own triangle) at the edges where it
+cannot: coincident and nearly coincident triangles, sheets closer than the FP32 bound, very small and very large
+triangles, lights that graze the surface.  Hit ids, t, shadow bits and the image must equal the oracle's."""
+import numpy as np
+import pytest
+
+from conftest import assert_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(n, z, jitter, rng):
+    """An n x n sheet of quads (two triangles each) facing the camera."""
+    t = np.linspace(-1.0, 1.0, n + 1)
+    x, y = np.meshgrid(t, t, indexing="ij")
+    p = np.stack([x, y, np.full_like(x, z)], -1) + rng.normal(0.0, jitter, x.shape + (3,))
+    a, b, c, d = p[:-1, :-1], p[1:, :-1], p[1:, 1:], p[:-1, 1:]
+    return np.concatenate([np.stack([a, b, c], 2).reshape(-1, 3, 3), np.stack([a, c, d], 2).reshape(-1, 3, 3)])
+
+
+def _scene(kind):
+    rng = np.random.default_rng(11)
+    if kind == "duplicates":
+        return np.repeat(_grid(12, -3.0, 0.05, rng), 3, 0)
+    if kind == "sheets":  # closer together than FP32 can tell
+        return np.concatenate([_grid(12, -3.0 - 1e-7 * k, 0.0, rng) for k in range(4)])
+    if kind == "crossing":  # two sheets that cut each other at a shallow angle
+        a, b = _grid(15, -3.0, 0.0, rng), _grid(15, -3.0, 0.0, rng)
+        a[..., 2] += 1e-4 * a[..., 0]
+        b[..., 2] -= 1e-4 * b[..., 0]
+        return np.concatenate([a, b])
+    if kind == "fine":
+        return _grid(160, -3.0, 1e-4, rng)
+    if kind == "coarse":
+        return _grid(1, -3.0, 0.0, rng) * np.array([40.0, 40.0, 1.0])
+    return _grid(12, -3.0, 0.02, rng) * 1e3  # large coordinates
+
+
+@pytest.mark.parametrize("kind", ["duplicates", "sheets", "crossing", "fine", "coarse", "large"])
+@pytest.mark.parametrize("light", [(2.5, 2.5, -0.5), (5.0, 0.5, -2.5), (5.0, 0.5, -2.4999999), (0.5, 0.5, -9.5)])
+@pytest.mark.parametrize("fstop", [np.inf, 2.0])
+def test_sure_hits(cuda, kind, light, fstop):
+    import crt
+    from crt import data
+    from oracle.oracle import OracleScene
+    v = _scene(kind).reshape(-1, 3).astype(np.float32)
+    n = len(v) // 3
+    idx = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    nrm = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (3 * n, 1))
+    m = data.Mesh(v, idx, nrm, idx.copy(), np.zeros(n, np.int32), data.lambert_material()[None])
+    cam = data.Camera(fov=50.0, focal_point=3.0, fstop=fstop)
+    lt = data.Light(position=light)
+    w, h, spp = 72, 52, 4
+    g, o = crt.Scene(m), OracleScene(m)
+    got = g.render(cam, lt, w, h, spp, aux=True, rays=True)
+    ref = o.render(cam, lt, w, h, spp=spp, aux=True, rays_in=got["rays"])
+    for k in ("hit_id", "hit_t", "shadow"):
+        assert_equal(got[k], ref[k], k)
+    assert_equal(got["rgb8"], ref["rgb"], "image")
+    b = crt.Batch([m], [(cam, lt, w, h, spp)])
+    assert_equal(b.run(np.zeros((w * h, 3), np.uint8)), got["rgb8"], "batched image")
+    g.check()
