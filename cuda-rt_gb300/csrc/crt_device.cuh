@@ -255,11 +255,19 @@ static __device__ __noinline__ bool box_exact(double ox, double oy, double oz, d
 
 // Certain rejection for the triangle test (tri_exact): true only when the
 // double Moller-Trumbore test certainly rejects.  The FP32 determinant and
-// numerators differ from the exact values by at most
-//   E_det = K |AB| |d| |AC|,  E_a = K |d| |AC| (|o| + |T|),
-//   E_b = K |d| |AB| (|o| + |T|)            (max-norms, K = 2^-16),
-// a factor of about 2^2 over a first-order rounding analysis with u = 2^-24
-// (the double computation's own error is far smaller).
+// numerators differ from the exact values by at most, in max-norms and to first
+// order in u = 2^-24 (inputs rounded to float, each product, difference and sum
+// rounded: 8u for a component of the cross products, 36u for the three products
+// of a dot product and 10u for its sums),
+//   46u |AB| |d| |AC|  (det),  46u |d| |AC| |T| + 6u |d| |AC| |o|  (alpha),
+//   46u |d| |AB| |T| + 6u |d| |AB| |o|  (beta).
+// The bounds used take 64u for 46u and 8u for 6u,
+//   E_det = K |AB| |d| |AC|,  E_a = K |d| |AC| (|T| + |o| / 8),
+//   E_b = K |d| |AB| (|T| + |o| / 8),  K = 2^-18,
+// which covers the second order and the double computation's own error.  (With
+// K = 2^-16 and |o| in place of |o| / 8, four to eight times the candidates were
+// left to exact tests: large frame 13.6 ms against 10.8, recursive 13.8 against
+// 12.4, 500k any-hit rays 435 us against 386.)
 //
 // self: the triangle that a shadow ray starts on (-1: none).  Its start is a
 // primary ray's hit, whose origin's components are at most r.oself, so its
@@ -286,8 +294,8 @@ __device__ __forceinline__ bool tri_reject_sure(const RayC& r, float4 a, float4 
   const float nAC = fmaxf(fmaxf(fabsf(ACx), fabsf(ACy)), fabsf(ACz));
   const float nT = fmaxf(fmaxf(fabsf(Tx), fabsf(Ty)), fabsf(Tz));
   const float nd = fmaxf(fmaxf(fabsf(r.fdx), fabsf(r.fdy)), fabsf(r.fdz));
-  const float K = 1.52587890625e-05f;  // 2^-16
-  const float ot = __fadd_ru(r.omax, nT);
+  const float K = 3.814697265625e-06f;  // 2^-18
+  const float ot = __fadd_ru(nT, 0.125f * r.omax);
   const float Ed = __fmul_ru(__fmul_ru(__fmul_ru(K, nAB), nd), nAC);
   const float Ea = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAC), ot);
   const float Eb = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAB), ot);
@@ -295,7 +303,7 @@ __device__ __forceinline__ bool tri_reject_sure(const RayC& r, float4 a, float4 
   if (__fadd_ru(ad, Ed) < 0.99e-8f) return true;  // |det| < 1e-8 for certain
   if (!(ad > Ed)) return false;                  // sign of det not certain
   if (self == __float_as_int(a.w) &&
-      __fsub_rd(ad, Ed) > __fmul_ru(__fmul_ru(__fmul_ru(1.2207031e-4f, nAB), nAC), __fadd_ru(ot, r.omax + r.oself)))
+      __fsub_rd(ad, Ed) > __fmul_ru(__fmul_ru(__fmul_ru(1.2207031e-4f, nAB), nAC), __fadd_ru(nT, 2.f * r.omax + r.oself)))
     return true;
   const float A = det > 0.f ? an : -an, Bv = det > 0.f ? bn : -bn;
   const float Dhi = __fmul_ru(__fadd_ru(ad, Ed), 1.0000001f);
@@ -310,7 +318,7 @@ __device__ __forceinline__ bool tri_reject_sure(const RayC& r, float4 a, float4 
 // What FP32 can say about the exact leaf test (box_exact and tri_exact):
 // kReject and kAccept are certain, kUnsure is neither.  With kAccept the exact
 // t lies in [lo, hi].  The bounds are tri_reject_sure's, with the numerator of
-// t bounded alike, E_t = K |AC| |AB| (|o| + |T|); t0 = tn / det from an
+// t bounded alike, E_t = K |AC| |AB| (|T| + |o| / 8); t0 = tn / det from an
 // approximate reciprocal is within (E_t + |t0| E_det) / (|det| - E_det) of the
 // exact t, and E_det <= |det| / 16 makes that at most 1.07 (..) / |det|; 1.1
 // and 2^-20 |t0| cover the FP32 roundings.  box: the box's test is certain too.
@@ -333,8 +341,8 @@ __device__ __forceinline__ TriClass tri_class(const RayC& r, float4 a, float4 b,
   const float nAC = fmaxf(fmaxf(fabsf(ACx), fabsf(ACy)), fabsf(ACz));
   const float nT = fmaxf(fmaxf(fabsf(Tx), fabsf(Ty)), fabsf(Tz));
   const float nd = fmaxf(fmaxf(fabsf(r.fdx), fabsf(r.fdy)), fabsf(r.fdz));
-  const float K = 1.52587890625e-05f;  // 2^-16
-  const float ot = __fadd_ru(r.omax, nT);
+  const float K = 3.814697265625e-06f;  // 2^-18
+  const float ot = __fadd_ru(nT, 0.125f * r.omax);
   const float Ed = __fmul_ru(__fmul_ru(__fmul_ru(K, nAB), nd), nAC);
   const float Ea = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAC), ot);
   const float Eb = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAB), ot);
@@ -614,8 +622,7 @@ __device__ __forceinline__ void cswap(float& ta, int& ca, float& tb, int& cb) {
 // are taken at once, and the lane walks on with their bound; of two whose t
 // intervals overlap, and of the uncertain ones, the exact test decides as
 // before, and the hit that remains takes one exact test at the end, all lanes
-// together.  Any hits take their exact tests as soon as kAnyVote lanes wait.
-// On soups, whose rays leave their warp, that ends most of the waiting
+// together.  On soups, whose rays leave their warp, that ends most of the waiting
 // (100,000 triangles 640x480x1: 859 -> 706 us; the 24-mesh batch 21.6 -> 15.0
 // ms); on the large sphere, whose rays stay together, little changes (13.78 ->
 // 13.68 ms).  The recursive kernel is 7% slower with it and leaves it out.
@@ -624,7 +631,6 @@ __device__ __forceinline__ void cswap(float& ta, int& ca, float& tb, int& cb) {
 // RAY_EPSILON), with h.id set; 0 otherwise.
 // NC = true reads the nodes and leaf triangles through the read-only cache;
 // NC = false uses ordinary (coherent) global loads, cached in L1 as well.
-constexpr int kAnyVote = 16;
 template <bool NC>
 __device__ __forceinline__ float4 ld_node(const float4* p) {
   if (NC) return __ldg(p);
@@ -667,7 +673,6 @@ __device__ __forceinline__ int traverse(const DScene& S, const RayC& r, const fl
     // FP32 phase: this lane's next candidate, a step of every walking lane per
     // round (the vote also brings the lanes together again)
     while (__any_sync(0xffffffffu, run && !pending)) {
-      if (SURE && ANY && __popc(__ballot_sync(0xffffffffu, pending)) >= kAnyVote) break;
       if (run && !pending) {
         bool got = node != kPop;
         while (!got && stk.sp > 0) {

@@ -60,3 +60,37 @@ def test_sure_hits(cuda, kind, light, fstop):
     b = crt.Batch([m], [(cam, lt, w, h, spp)])
     assert_equal(b.run(np.zeros((w * h, 3), np.uint8)), got["rgb8"], "batched image")
     g.check()
+
+
+@pytest.mark.parametrize("scale", [1e-3, 1.0, 1e3])
+@pytest.mark.parametrize("offset", [0.0, 30.0, 3e4])
+def test_rays_at_edges(cuda, scale, offset):
+    """Rays aimed at edges and corners, on them and beside them by 1e-9 to 1e-4 of a triangle: the FP32 filters'
+    error bounds decide which of these take the exact test; closest and any hits must be the oracle's."""
+    import crt
+    from crt import data
+    from oracle.oracle import OracleScene
+    rng = np.random.default_rng(3)
+    tri = _grid(14, 0.0, 0.02, rng)
+    v = (tri.reshape(-1, 3) * scale + offset).astype(np.float32)
+    n = len(v) // 3
+    idx = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    nrm = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (3 * n, 1))
+    m = data.Mesh(v, idx, nrm, idx.copy(), np.zeros(n, np.int32), data.lambert_material()[None])
+    g, o = crt.Scene(m), OracleScene(m)
+    k = 12_000
+    t = v.reshape(-1, 3, 3).astype(np.float64)[rng.integers(0, n, k)]
+    s = np.where(rng.random(k) < 0.2, 0.0, rng.random(k))[:, None]  # corners, points of edges
+    p = t[:, 0] + s * (t[:, 1] - t[:, 0])
+    size = np.linalg.norm(t[:, 1] - t[:, 0], axis=1, keepdims=True)
+    p = p + rng.normal(size=(k, 3)) * size * 10.0 ** rng.uniform(-9, -4, (k, 1)) * (rng.random((k, 1)) < 0.8)
+    d = rng.normal(size=(k, 3))
+    d[: k // 4, 2] *= 1e-3  # grazing
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.hstack([p - d * scale * rng.uniform(0.0, 4.0, (k, 1)), d])
+    for any_hit in (False, True):
+        gi, gt = g.trace(rays, any_hit=any_hit)
+        oi, ot, _ = o.trace(rays, any_hit=any_hit)
+        assert_equal(gi, oi, f"ids any={any_hit}")
+        assert_equal(gt, ot, f"t any={any_hit}")
+    g.check()
