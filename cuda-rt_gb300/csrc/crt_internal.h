@@ -150,6 +150,7 @@ constexpr int kMinTilesPerRegion = 256;
 struct RenderArgs {
   int W, H, spp, row0, row1;
   int group;  // lanes per pixel (lanes_per_pixel)
+  int tile_w = 0, tile_h = 0;  // pixels of a tile (spread_pixels; at most 32 / group)
   int regions_x = 1, regions_y = 1;  // tile rectangles (set_tile_regions); counter holds one word per rectangle
   double angle, aspect, invW, invH, aperture, focal;
   double eye[3];
@@ -177,11 +178,12 @@ struct RenderArgs {
 };
 cudaError_t launch_render(const DScene& S, const RenderArgs& a, cudaStream_t st);
 
-
 // The tile rectangles for a tiles_x x tiles_y grid of tiles: with split and a
 // large enough image about num_sms() of them, near square, else one; their
 // counters and bound zeroed on st.
 cudaError_t set_tile_regions(RenderArgs& a, int tiles_x, int tiles_y, bool split, cudaStream_t st);
+// Sets the tile of a frame, and for few pixels raises its lanes per pixel to at most gmax.
+void spread_pixels(RenderArgs& a, int gmax);
 
 // lens.cu: the thin-lens tables of the current device (built on first use
 // when enabled and memory allows; otherwise both NULL, and the kernels

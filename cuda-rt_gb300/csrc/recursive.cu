@@ -35,7 +35,8 @@ namespace {
 // when spp is smaller): on the depth-3 mirror/glass frame (1280x720, 4 spp)
 // 2 lanes took 16.0 ms, 4 lanes 18.3 ms (more walks start from wrong guesses)
 // and 1 lane 19.0 ms.  Without secondary rays (depth 0) one lane per pixel
-// is fastest (3.3 against 3.5 ms): there is no tree to overlap.
+// is fastest (3.3 against 3.5 ms): there is no tree to overlap.  Small images
+// take up to four (spread_pixels).
 constexpr int kRecLanesPerPixel = 2;
 
 struct Frame {
@@ -131,13 +132,15 @@ __device__ __forceinline__ PixelRay primary(const RenderArgs& A, D3 fdir, uint32
 // The tree of a sample is walked depth first with an explicit frame stack,
 // as the recursion of traceRay; every step traces the next ray of every lane
 // that has one, then the shadow rays of the lanes whose ray hit.
-__global__ void __launch_bounds__(128) k_pixels_rec(DScene S, RenderArgs A, const DOptics* __restrict__ optics,
+// Three blocks of 168 registers per SM: more warps spill what their long walks
+// keep (4 blocks 12.1 ms, 5 12.0 to 12.4, 6 13.0, 2 with 222 registers 13.1; 3: 11.9).
+__global__ void __launch_bounds__(128, 3) k_pixels_rec(DScene S, RenderArgs A, const DOptics* __restrict__ optics,
                                                     int depth) {
   const unsigned full = 0xffffffffu;
   float rb[6], B, D;
   scene_consts(S, rb, B, D);
   const int lane = threadIdx.x & 31;
-  const int G = A.group, tw = group_tile_w(G), th = group_tile_h(G);
+  const int G = A.group, tw = A.tile_w, th = A.tile_h;
   const int g = lane & (G - 1);
   const int base = lane - g;
   const unsigned gmask = (G == 32) ? full : (((1u << G) - 1u) << base);
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(128) k_pixels_rec(DScene S, RenderArgs A, cons
     const int pp = lane / G;  // this lane's pixel in the tile
     const int tx = (tile % tiles_x) * tw, ty = A.row0 + (tile / tiles_x) * th;
     const int px = tx + (pp % tw), py = ty + (pp / tw);
-    const bool valid = px < A.W && py < A.row1;
+    const bool valid = pp < tw * th && px < A.W && py < A.row1;
     if (!A.rays && beam_misses(S, A, rb, B, tx, tx + tw - 1, ty, ty + th - 1)) {
       write_miss<kRender>(A, px, py, valid, G, miss_mean(A.spp));
       if (valid && g == 0) nrays += (unsigned)A.spp;
@@ -359,7 +362,8 @@ cudaError_t launch_render_recursive(const DScene& S, const RenderArgs& a, const 
   if (depth < 0 || depth > kMaxRecDepth) return cudaErrorInvalidValue;
   RenderArgs r = a;
   r.group = depth > 0 ? lanes_per_pixel(a.spp, kRecLanesPerPixel) : 1;
-  const int tw = group_tile_w(r.group), th = group_tile_h(r.group);
+  spread_pixels(r, 4);
+  const int tw = r.tile_w, th = r.tile_h;
   // (one rectangle: the cost of a pixel's ray trees varies too much for rectangles of equal size)
   cudaError_t e = set_tile_regions(r, (r.W + tw - 1) / tw, (r.row1 - r.row0 + th - 1) / th, false, st);
   if (e != cudaSuccess) return e;

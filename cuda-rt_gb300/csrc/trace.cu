@@ -7,7 +7,7 @@
 //               traceRay (raytracer.cu:169-249), Material::shade
 //               (kernels/material.cu:6-40) and the positional Light
 //               (kernels/Light.cu:5-86); also its adjoint.  Persistent: each
-//               warp claims tiles of 32 / G pixels (G lanes per pixel), first
+//               warp claims tiles of at most 32 / G pixels (G lanes per pixel), first
 //               from its SM's rectangle of the image, then from the others;
 //               a pixel's lanes trace its samples in waves, speculating on
 //               how the mrand stream couples them (a hit consumes three
@@ -60,11 +60,12 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ DScene
       });
 }
 
-// One scene: warps claim tiles of 32 / G pixels of rows [row0, row1).
+// One scene: warps claim tiles of tile_w x tile_h pixels (at most 32 / G) of
+// rows [row0, row1).  BPS: blocks per SM (launch_render).
 // SHORT: traversal-stack entries kept in shared memory per thread.
 constexpr int kPixelsShort = 0;
-template <int MODE>
-__global__ void __launch_bounds__(128, 9) k_pixels(DScene S, RenderArgs A) {
+template <int MODE, int BPS>
+__global__ void __launch_bounds__(128, BPS) k_pixels(DScene S, RenderArgs A) {
   extern __shared__ int2 s_ring[];
   int2* ring = kPixelsShort > 0 ? s_ring + threadIdx.x : nullptr;
   TravStats ts;
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(128, 9) k_pixels(DScene S, RenderArgs A) {
   float rb[6], B, D;
   scene_consts(S, rb, B, D);
   const int lane = threadIdx.x & 31;
-  const int G = A.group, tw = group_tile_w(G), th = group_tile_h(G);
+  const int G = A.group, tw = A.tile_w, th = A.tile_h;
   const int tiles_x = (A.W + tw - 1) / tw;
   const int tiles_y = (A.row1 - A.row0 + th - 1) / th;
   const int p = lane / G;  // this lane's pixel in the tile
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(128, 9) k_pixels(DScene S, RenderArgs A) {
     if (tile < 0) break;
     const int tx = (tile % tiles_x) * tw, ty = A.row0 + (tile / tiles_x) * th;
     const int px = tx + (p % tw), py = ty + (p / tw);
-    const bool valid = px < A.W && py < A.row1;
+    const bool valid = p < tw * th && px < A.W && py < A.row1;
     if (cull && beam_misses(S, A, rb, B, tx, tx + tw - 1, ty, ty + th - 1)) {
       if (miss == 0.0) miss = miss_mean(A.spp);
       write_miss<MODE>(A, px, py, valid, G, miss);
@@ -101,12 +102,12 @@ __global__ void __launch_bounds__(128, 9) k_pixels(DScene S, RenderArgs A) {
 
 }  // namespace
 
-template <int MODE>
+template <int MODE, int BPS>
 static void launch_pixels(const DScene& S, const RenderArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)kPixelsShort * 128 * sizeof(int2);
   int bps = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_pixels<MODE>, 128, smem);
-  k_pixels<MODE><<<num_sms() * (bps > 0 ? bps : 1), 128, smem, st>>>(S, a);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_pixels<MODE, BPS>, 128, smem);
+  k_pixels<MODE, BPS><<<num_sms() * (bps > 0 ? bps : 1), 128, smem, st>>>(S, a);
 }
 
 cudaError_t set_tile_regions(RenderArgs& a, int tiles_x, int tiles_y, bool split, cudaStream_t st) {
@@ -123,17 +124,53 @@ cudaError_t set_tile_regions(RenderArgs& a, int tiles_x, int tiles_y, bool split
   return cudaMemsetAsync(a.counter, 0, sizeof(unsigned) * (size_t)(rx * ry + 1), st);
 }
 
+// Images of few pixels: what bounds them is not throughput but the slowest
+// warp, so their work is spread over more warps.
+//  - More lanes per pixel (up to gmax: fewer waves one after another) while
+//    that leaves fewer than 288 / G warps' worth of lanes per SM (36 are
+//    resident; with more lanes more samples start from wrong guesses).
+//    100,000-triangle soup at 16 samples, 4 lanes against the rule's up to 16:
+//    160x120 1035 -> 470 us, 320x240 1524 -> 1287; 7,080-triangle sphere, 64x48
+//    530 -> 515, 240x180 1013 -> 790, 320x240 1096 -> 1060 (16 lanes there:
+//    1105).  Depth-3 recursion at 4 samples, 2 lanes against up to 4: 640x360
+//    7.7 -> 6.8 ms, 320x180 6.4 -> 5.5.
+//  - Tiles of fewer pixels than a warp holds until every SM has 24 (the lanes
+//    left over only vote): fewer different walks wait for one another.
+//    2,000 triangles, 64x48 at 2 samples, with the build: 119 -> 100 us (12 per
+//    SM 104, 16 to 36 100); 72 slow down 640x480 at one sample, 645 -> 800.
+//    Recursion: 160x90 6.3 -> 4.0 ms (16 per SM 4.4), 64x48 5.5 -> 2.1.
+void spread_pixels(RenderArgs& a, int gmax) {
+  const int rows = a.row1 - a.row0;
+  const int64_t sms = num_sms(), px = (int64_t)a.W * rows;
+  while (2 * a.group <= min(a.spp, gmax) && px * a.group * a.group < 288 * 32 * sms) a.group *= 2;
+  int tw = group_tile_w(a.group), th = group_tile_h(a.group);
+  while (tw * th > 1 && (int64_t)((a.W + tw - 1) / tw) * ((rows + th - 1) / th) < 24 * sms) {
+    if (tw >= th)
+      tw /= 2;
+    else
+      th /= 2;
+  }
+  a.tile_w = tw, a.tile_h = th;
+}
+
 cudaError_t launch_render(const DScene& S, const RenderArgs& a0, cudaStream_t st) {
   RenderArgs a = a0;
-  const int tw = group_tile_w(a.group), th = group_tile_h(a.group);
-  cudaError_t e = set_tile_regions(a, (a.W + tw - 1) / tw, (a.row1 - a.row0 + th - 1) / th, true, st);
+  spread_pixels(a, 16);
+  const int tiles_x = (a.W + a.tile_w - 1) / a.tile_w, tiles_y = (a.row1 - a.row0 + a.tile_h - 1) / a.tile_h;
+  cudaError_t e = set_tile_regions(a, tiles_x, tiles_y, true, st);
   if (e != cudaSuccess) return e;
+  // Nine blocks of 56 registers per SM, but seven of 72 below two tiles per
+  // resident warp, where the warps' own time counts: 640x480 soup at one sample
+  // 648 -> 600 us, 320x240 at 4 604 -> 585; above it 400x300 at 4 (99 tiles per
+  // SM) is 752 us with nine against 777, the large frame 11.0 ms against 11.4.
   if (a.grad_rgb)
-    launch_pixels<kAdjoint>(S, a, st);
+    launch_pixels<kAdjoint, 9>(S, a, st);
   else if (a.stats)
-    launch_pixels<kRenderStats>(S, a, st);
+    launch_pixels<kRenderStats, 9>(S, a, st);
+  else if ((int64_t)tiles_x * tiles_y < 72 * num_sms())
+    launch_pixels<kRender, 7>(S, a, st);
   else
-    launch_pixels<kRender>(S, a, st);
+    launch_pixels<kRender, 9>(S, a, st);
   return cudaGetLastError();
 }
 
