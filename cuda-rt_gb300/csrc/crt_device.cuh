@@ -129,7 +129,7 @@ struct RayC {
   float dprune;          // widening of the entry bound for pruning
   float tau;             // slack on t for pruning
   int sx, sy, sz;        // 1 when 1/d < 0: the box's hi plane is the near one
-  float oself;           // see tri_class (set by callers that name the ray's own triangle)
+  float oself;           // see tri_reject_sure (set by callers that name the ray's own triangle)
 };
 
 // The largest scene coordinate the slab filter works with; beyond it every axis
@@ -209,16 +209,21 @@ __device__ __forceinline__ bool box_cons(const RayC& r, float lox, float hix, fl
   return L <= U;
 }
 
-// Certain acceptance: true only when box_exact is certainly true (every
-// exact entry value <= every exact exit value).
+// Certain acceptance: true only when box_exact is certainly true (every exact
+// entry value <= every exact exit value).  On one axis the entry never exceeds
+// the exit: (lo - o) and (hi - o) round in order, and so do their products
+// with 1/d (finite, on an axis that is not free).  So only different axes are
+// compared, and the flat box of an axis-aligned triangle can be certain
+// too: without that every hit of a floor or wall took the double box test
+// (three divisions) as well.
 __device__ __forceinline__ bool box_sure(const RayC& r, float lox, float hix, float loy, float hiy, float loz,
                                          float hiz) {
   const float nx = r.sx ? hix : lox, fx = r.sx ? lox : hix;
   const float ny = r.sy ? hiy : loy, fy = r.sy ? loy : hiy;
   const float nz = r.sz ? hiz : loz, fz = r.sz ? loz : hiz;
-  const float L = fmaxf(fmaxf(__fmaf_ru(nx, r.ax, r.hx), __fmaf_ru(ny, r.ay, r.hy)), __fmaf_ru(nz, r.az, r.hz));
-  const float U = fminf(fminf(__fmaf_rd(fx, r.ax, r.lx), __fmaf_rd(fy, r.ay, r.ly)), __fmaf_rd(fz, r.az, r.lz));
-  return L <= U;
+  const float Lx = __fmaf_ru(nx, r.ax, r.hx), Ly = __fmaf_ru(ny, r.ay, r.hy), Lz = __fmaf_ru(nz, r.az, r.hz);
+  const float Ux = __fmaf_rd(fx, r.ax, r.lx), Uy = __fmaf_rd(fy, r.ay, r.ly), Uz = __fmaf_rd(fz, r.az, r.lz);
+  return Lx <= fminf(Uy, Uz) && Ly <= fminf(Ux, Uz) && Lz <= fminf(Ux, Uy);
 }
 
 // BoundingBox::intersect(const ray&), inc/bbox.h:82-102, in double.  Kept
@@ -269,14 +274,15 @@ static __device__ __noinline__ bool box_exact(double ox, double oy, double oz, d
 // left to exact tests: large frame 13.6 ms against 10.8, recursive 13.8 against
 // 12.4, 500k any-hit rays 435 us against 386.)
 //
-// self: the triangle that a shadow ray starts on (-1: none).  Its start is a
-// primary ray's hit, whose origin's components are at most r.oself, so its
+// self: the triangle that a shadow or secondary ray starts on (-1: none).  Its
+// start is a ray's hit, and the components of that ray's origin are at most r.oself, so its
 // exact t is rounding alone: with u = 2^-53 and M = |o_primary| + |o| + |A| +
 // |T|, the start lies off the plane by less than 2^8 u |AB| |AC| M (in units of
 // the numerator of t), |t| < 2^9 u |AB| |AC| M / |det|, and the exact test
 // certainly rejects it (|t| < 1e-8) when |det| > 2^-17.4 |AB| |AC| M; 2^-13 is
-// used.  Every shadow ray meets its own triangle: without this it took one of
-// its two exact tests for it.
+// used.  Every such ray meets its own triangle: without this it took one of
+// its two exact tests for it (depth-3 recursion 11.9 -> 11.2 ms with it for the
+// shadow rays, 10.95 with it for the secondary rays too).
 __device__ __forceinline__ bool tri_reject_sure(const RayC& r, float4 a, float4 b, float4 c, int self = -1) {
   const float ABx = b.x - a.x, ABy = b.y - a.y, ABz = b.z - a.z;
   const float ACx = c.x - a.x, ACy = c.y - a.y, ACz = c.z - a.z;
@@ -725,7 +731,7 @@ __device__ __forceinline__ int traverse(const DScene& S, const RayC& r, const fl
           if constexpr (SURE && !ANY)
             k = tri_class(r, a, b, c, lo, hi, box);
           else
-            k = tri_reject_sure(r, a, b, c, ANY ? self : -1) ? kReject : kUnsure;
+            k = tri_reject_sure(r, a, b, c, self) ? kReject : kUnsure;
           if (k != kReject) {
             // the leaf's box (as the refit computes it from the same vertices)
             // is tested here rather than when the leaf is pushed: one copy of

@@ -43,6 +43,8 @@ struct Frame {
   D3 c;        // colour so far: shade(), then each child's contribution
   D3 q, N, d;  // hit point, smooth normal, incoming direction
   int mid;     // material
+  int id;      // triangle
+  float omax;  // the bound of the ray's origin (RayC)
   int stage;   // 0 no child yet, 1 reflected child out, 2 refracted child out, 3 done
 };
 
@@ -201,6 +203,8 @@ __global__ void __launch_bounds__(128, 3) k_pixels_rec(DScene S, RenderArgs A, c
         uint32_t st = wst;
         int lvl = 0;
         PixelRay ray{d3(0, 0, 0), d3(0, 0, 1)};
+        int self = -1;  // the triangle that ray starts on, hit by a ray whose origin is bounded by oself
+        float oself = 0.f;
         if (busy) {
           for (int t = 0; t < off; t++) xorshift32(st);
           ray = primary(A, fdir, st);
@@ -213,8 +217,9 @@ __global__ void __launch_bounds__(128, 3) k_pixels_rec(DScene S, RenderArgs A, c
             ray_setup(rc, ray.org.x, ray.org.y, ray.org.z, ray.dir.x, ray.dir.y, ray.dir.z, B, D);
           else
             ray_setup(rc, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, B, D);
+          rc.oself = oself;
           HitRec h;
-          const int res = traverse<false>(S, rc, rb, h, busy);
+          const int res = traverse<false>(S, rc, rb, h, busy, nullptr, nullptr, 0.f, self);
           if (res < 0) atomicOr(&S.g->err, kErrStack);
           const bool hit = busy && res > 0;
           wr += busy, ws += hit, hits += hit;
@@ -234,7 +239,8 @@ __global__ void __launch_bounds__(128, 3) k_pixels_rec(DScene S, RenderArgs A, c
             ray_setup(sr, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, B, D);
           }
           HitRec sh;
-          const int sres = traverse<true>(S, sr, rb, sh, hit, nullptr, nullptr, (float)dist);
+          sr.oself = rc.omax;
+          const int sres = traverse<true>(S, sr, rb, sh, hit, nullptr, nullptr, (float)dist, hit ? h.id : -1);
           if (sres < 0) atomicOr(&S.g->err, kErrStack);
           if (!busy) continue;
           // Material::shade (kernels/material.cu:6-40), as the plain pixel kernel
@@ -269,8 +275,9 @@ __global__ void __launch_bounds__(128, 3) k_pixels_rec(DScene S, RenderArgs A, c
           // colour up the frames until one has another child or the tree ends
           if (hit && lvl < depth) {
             Frame& f = fr[lvl];
-            f.c = c, f.q = q, f.N = N, f.d = ray.dir, f.mid = mid, f.stage = 0;
+            f.c = c, f.q = q, f.N = N, f.d = ray.dir, f.mid = mid, f.id = h.id, f.omax = rc.omax, f.stage = 0;
             if (next_child(f, optics, S.mats, ray.org, ray.dir)) {
+              self = f.id, oself = f.omax;
               lvl++;
               continue;
             }
@@ -285,7 +292,10 @@ __global__ void __launch_bounds__(128, 3) k_pixels_rec(DScene S, RenderArgs A, c
             }
             Frame& f = fr[lvl - 1];
             add_child(f, optics, S.mats, c);
-            if (next_child(f, optics, S.mats, ray.org, ray.dir)) break;
+            if (next_child(f, optics, S.mats, ray.org, ray.dir)) {
+              self = f.id, oself = f.omax;
+              break;
+            }
             c = f.c;
             lvl--;
           }

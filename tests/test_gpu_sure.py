@@ -94,3 +94,45 @@ def test_rays_at_edges(cuda, scale, offset):
         assert_equal(gi, oi, f"ids any={any_hit}")
         assert_equal(gt, ot, f"t any={any_hit}")
     g.check()
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("offset", [0.0, 0.3, -700.0])
+def test_flat_boxes(cuda, axis, offset):
+    """Axis-aligned triangles, whose boxes are flat: rays inside, on and beside their edges, along the axis, across
+    it and within the plane."""
+    import crt
+    from crt import data
+    from oracle.oracle import OracleScene
+    rng = np.random.default_rng(7)
+    k = 8
+    lo = rng.uniform(-1.0, 0.5, (k, 2))
+    hi = lo + rng.uniform(0.1, 0.8, (k, 2))
+    quads = []
+    for j in range(k):
+        (a, b), (c, d) = lo[j], hi[j]
+        quads += [[(a, b), (c, b), (c, d)], [(a, b), (c, d), (a, d)]]
+    flat = np.repeat(rng.choice([-0.5, 0.0, 0.25, 0.25], k), 2)[:, None, None]
+    tri = np.concatenate([np.broadcast_to(flat, (2 * k, 3, 1)), np.asarray(quads)], 2)
+    v = (np.roll(tri, axis, axis=2).reshape(-1, 3) + offset).astype(np.float32)
+    n = len(v) // 3
+    idx = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    nrm = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (3 * n, 1))
+    m = data.Mesh(v, idx, nrm, idx.copy(), np.zeros(n, np.int32), data.lambert_material()[None])
+    g, o = crt.Scene(m), OracleScene(m)
+    count = 6_000
+    t = v.reshape(-1, 3, 3).astype(np.float64)[rng.integers(0, n, count)]
+    w = rng.dirichlet([0.5, 0.5, 0.5], count) * (rng.random((count, 3)) < 0.8)  # faces, edges and corners
+    w[w.sum(1) == 0] = (1.0, 0.0, 0.0)
+    p = np.einsum("ij,ijk->ik", w / w.sum(1, keepdims=True), t)
+    d = rng.normal(size=(count, 3))
+    d[: count // 4] *= np.array([1e-4, 1.0, 1.0])[[(c - axis) % 3 for c in range(3)]]  # grazing
+    d[count // 4: count // 3] = np.eye(3)[rng.integers(0, 3, count // 3 - count // 4)]  # along an axis
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.hstack([p - d * rng.uniform(0.0, 3.0, (count, 1)), d])
+    for any_hit in (False, True):
+        gi, gt = g.trace(rays, any_hit=any_hit)
+        oi, ot, _ = o.trace(rays, any_hit=any_hit)
+        assert_equal(gi, oi, f"ids any={any_hit}")
+        assert_equal(gt, ot, f"t any={any_hit}")
+    g.check()
