@@ -136,13 +136,33 @@ __device__ __forceinline__ bool beam_misses(const DScene& S, const RenderArgs& A
   return false;
 }
 
+// sum / spp: a power of two's inverse is exact, and so is the product's rounding.
+__device__ __forceinline__ double sample_mean(double sum, int spp) {
+  if ((spp & (spp - 1)) == 0) return sum * __hiloint2double((1023 - (31 - __clz(spp))) << 20, 0);
+  return sum / (double)spp;
+}
+
+// Lane j of every four lanes has a row v0..v3; afterwards it has column j.
+__device__ __forceinline__ void swap_if(bool p, double& a, double& b) {
+  const double t = p ? b : a;
+  b = p ? a : b;
+  a = t;
+}
+__device__ __forceinline__ void quad_transpose(double& v0, double& v1, double& v2, double& v3) {
+  const unsigned full = 0xffffffffu;
+  const bool b0 = threadIdx.x & 1, b1 = threadIdx.x & 2;
+  swap_if(b0, v0, v1), swap_if(b0, v2, v3), swap_if(b1, v0, v2), swap_if(b1, v1, v3);
+  v1 = __shfl_xor_sync(full, v1, 1), v2 = __shfl_xor_sync(full, v2, 2), v3 = __shfl_xor_sync(full, v3, 3);
+  swap_if(b0, v0, v1), swap_if(b0, v2, v3), swap_if(b1, v0, v2), swap_if(b1, v1, v3);
+}
+
 // The pixel this lane would have shaded, when the block's beam misses: every
 // sample is a miss.  mean: 0.9 summed spp times in double and divided by spp,
 // as the samples would be.
 __device__ __forceinline__ double miss_mean(int spp) {
   double a = 0.0;
   for (int i = 0; i < spp; i++) a = a + 0.9;
-  return a / (double)spp;
+  return sample_mean(a, spp);
 }
 
 // Writes a block's missing pixels (this lane's when it leads its group of G).
@@ -182,7 +202,9 @@ __device__ __forceinline__ void write_miss(const RenderArgs& A, int px, int py, 
 // majority), traces, and the lanes whose guess of an earlier sample proved
 // wrong trace again with the hits just observed; at least one more sample of
 // every group is settled per round, and the settled rays are exactly the
-// sequential ones.  Colours and depths are then summed in sample order.
+// sequential ones.  Colours and depths are then summed in sample order; with four
+// lanes or more each lane of four sums one of x, y, z and depth (an inactive
+// lane's zeros change no sum: none is ever -0).
 template <int MODE, int SHORT = 0, bool NC = true>
 __device__ __forceinline__ void pixel(const DScene& S, const RenderArgs& A, int px, int py, bool valid, int G,
                                       unsigned& pred, float rb[6], float B, float D, TravStats& ts, D3& glight,
@@ -418,24 +440,43 @@ __device__ __forceinline__ void pixel(const DScene& S, const RenderArgs& A, int 
         if (A.shadow_id) A.shadow_id[si] = shid;
       }
       // sum in sample order (the reference adds the samples one by one)
-      for (int t = 0; t < G; t++) {
-        const double cx = __shfl_sync(full, col.x, base + t), cy = __shfl_sync(full, col.y, base + t),
-                     cz = __shfl_sync(full, col.z, base + t);
-        const double dt = __shfl_sync(full, hit ? h.t : 0.0, base + t);
-        if (w * G + t < A.spp) {
-          acc = acc + d3(cx, cy, cz);
-          if ((hits >> (base + t)) & 1u) depth += dt;
+      if (MODE != kAdjoint) {
+        double v0 = act ? col.x : 0.0, v1 = act ? col.y : 0.0, v2 = act ? col.z : 0.0, v3 = hit ? h.t : 0.0;
+        if (G >= 4) {
+          quad_transpose(v0, v1, v2, v3);
+          for (int t = 0; t < G; t += 4) {
+            const int src = base + t + (lane & 3);
+            const double a0 = __shfl_sync(full, v0, src), a1 = __shfl_sync(full, v1, src),
+                         a2 = __shfl_sync(full, v2, src), a3 = __shfl_sync(full, v3, src);
+            acc.x = acc.x + a0;
+            acc.x = acc.x + a1;
+            acc.x = acc.x + a2;
+            acc.x = acc.x + a3;
+          }
+        } else {
+          for (int t = 0; t < G; t++) {
+            acc = acc + d3(__shfl_sync(full, v0, base + t), __shfl_sync(full, v1, base + t),
+                           __shfl_sync(full, v2, base + t));
+            depth += __shfl_sync(full, v3, base + t);
+          }
         }
       }
       // guess for the next wave: the group's majority
       const int nh = __popc(hits & gmask), na = __popc(actm & gmask);
       pred = __ballot_sync(full, 2 * nh >= na);
     }
-    if (MODE == kAdjoint || !valid || g != 0) return;
-    const double inv = (double)A.spp;
-    acc = d3(acc.x / inv, acc.y / inv, acc.z / inv);
+    if (MODE == kAdjoint) return;
+    if (G >= 4) {
+      const double m = sample_mean(acc.x, A.spp);
+      acc = d3(m, __shfl_sync(full, m, base + 1), __shfl_sync(full, m, base + 2));
+      depth = __shfl_sync(full, m, base + 3);
+    } else {
+      acc = d3(sample_mean(acc.x, A.spp), sample_mean(acc.y, A.spp), sample_mean(acc.z, A.spp));
+      depth = sample_mean(depth, A.spp);
+    }
+    if (!valid || g != 0) return;
     write_pixel(A, idx, acc);
-    if (A.depth) A.depth[idx] = depth / inv;
+    if (A.depth) A.depth[idx] = depth;
 }
 
 template <int MODE>
