@@ -677,50 +677,17 @@ __device__ __forceinline__ int traverse(const DScene& S, const RayC& r, const fl
   int steps = 0;
   while (true) {
     // FP32 phase: this lane's next candidate, a step of every walking lane per
-    // round (the vote also brings the lanes together again)
+    // round (the vote also brings the lanes together again).  A step tests the
+    // leaf in hand, if any, and goes on to a node: most rounds run both parts
+    // for some lane anyway, and a lane with a leaf need not sit out the nodes'
+    // (one or the other per step: 24-mesh batch 13.3 ms against 12.45, large
+    // frame 10.87 against 10.42, recursion 10.4 against 10.1; waiting for eight
+    // lanes with leaves 15.2, 11.3 and 11.9)
     while (__any_sync(0xffffffffu, run && !pending)) {
-      if (run && !pending) {
-        bool got = node != kPop;
-        while (!got && stk.sp > 0) {
-          const E e = stk.pop();
-          if (ANY || !(entry_bound(e) > pb)) node = entry_node(e), got = true;
-        }
-        if (!got) {
-          run = false;
-        } else if (++steps > max_steps || node >= S.ntri - 1 || (node < 0 && (~node & kLeafIndex) >= S.ntri) ||
-                   stk.sp > kWideStack - 4) {  // only a corrupt tree gets here
+      if (run && !pending && node < 0 && node != kPop) {
+        if (++steps > max_steps || (~node & kLeafIndex) >= S.ntri) {  // only a corrupt tree gets here
           err = true;
           run = false;
-        } else if (node >= 0) {
-          if (STATS) ts->nodes++;
-          float L[4], U[4];
-          int c[4];
-          load_slabs<NC>(S.wnodes + node, r, L, U, c);
-          node = kPop;
-          if (ANY) {
-            // the first hit slot is next, the others are stacked so they pop in order
-#pragma unroll
-            for (int k = 3; k >= 0; k--) {
-              if (L[k] <= U[k] && c[k] != kNoChild) {
-                if (node != kPop) stk.push(stack_entry(node, 0.f, (E*)nullptr));
-                node = c[k];
-              }
-            }
-          } else {
-            // nearest first; misses (+inf) sort last
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-              if (!(L[k] <= fminf(U[k], pb) && c[k] != kNoChild)) c[k] = kNoChild, L[k] = __int_as_float(0x7f800000);
-            cswap(L[0], c[0], L[1], c[1]);
-            cswap(L[2], c[2], L[3], c[3]);
-            cswap(L[0], c[0], L[2], c[2]);
-            cswap(L[1], c[1], L[3], c[3]);
-            cswap(L[1], c[1], L[2], c[2]);
-#pragma unroll
-            for (int k = 3; k >= 1; k--)
-              if (c[k] != kNoChild) stk.push(stack_entry(c[k], L[k], (E*)nullptr));
-            node = c[0];
-          }
         } else {
           if (STATS) ts->tris++;
           const float4* lp = reinterpret_cast<const float4*>(S.leaves + (~node & kLeafIndex));
@@ -750,7 +717,52 @@ __device__ __forceinline__ int traverse(const DScene& S, const RayC& r, const fl
             }
             if (open) cand = box ? node : ~(~node | kLeafBoxDue), pending = true;
           }
-          node = kPop;
+        }
+        node = kPop;
+      }
+      if (run && !pending) {
+        bool got = node != kPop;
+        while (!got && stk.sp > 0) {
+          const E e = stk.pop();
+          if (ANY || !(entry_bound(e) > pb)) node = entry_node(e), got = true;
+        }
+        if (!got) {
+          run = false;
+        } else if (node >= 0) {
+          if (++steps > max_steps || node >= S.ntri - 1 || stk.sp > kWideStack - 4) {  // only a corrupt tree gets here
+            err = true;
+            run = false;
+          } else {
+            if (STATS) ts->nodes++;
+            float L[4], U[4];
+            int c[4];
+            load_slabs<NC>(S.wnodes + node, r, L, U, c);
+            node = kPop;
+            if (ANY) {
+              // the first hit slot is next, the others are stacked so they pop in order
+#pragma unroll
+              for (int k = 3; k >= 0; k--) {
+                if (L[k] <= U[k] && c[k] != kNoChild) {
+                  if (node != kPop) stk.push(stack_entry(node, 0.f, (E*)nullptr));
+                  node = c[k];
+                }
+              }
+            } else {
+              // nearest first; misses (+inf) sort last
+#pragma unroll
+              for (int k = 0; k < 4; k++)
+                if (!(L[k] <= fminf(U[k], pb) && c[k] != kNoChild)) c[k] = kNoChild, L[k] = __int_as_float(0x7f800000);
+              cswap(L[0], c[0], L[1], c[1]);
+              cswap(L[2], c[2], L[3], c[3]);
+              cswap(L[0], c[0], L[2], c[2]);
+              cswap(L[1], c[1], L[3], c[3]);
+              cswap(L[1], c[1], L[2], c[2]);
+#pragma unroll
+              for (int k = 3; k >= 1; k--)
+                if (c[k] != kNoChild) stk.push(stack_entry(c[k], L[k], (E*)nullptr));
+              node = c[0];
+            }
+          }
         }
       }
     }
