@@ -210,9 +210,9 @@ __global__ void __launch_bounds__(TH, 1) k_sort_coop(const uint32_t* kin0, const
                                                      uint32_t* counts, unsigned* bar, int* err) {
   constexpr int W = TH / 32;
   constexpr int TILE = TH * IT;
-  constexpr int DPT = kRadix / TH;
-  static_assert(kRadix % TH == 0 && 32 * IT < 65536, "digits per thread, 16-bit warp counters");
+  static_assert(TH == kRadix && TILE <= 8192, "one digit per thread, 16-bit sums of four counts");
   __shared__ SortSmem<TH, IT> sm;
+  __shared__ __align__(16) uint32_t s_part[2][4][kRadix];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tile = blockIdx.x, ntiles = gridDim.x, base = tile * TILE;
   const uint32_t mask = kRadix - 1;
@@ -256,60 +256,52 @@ __global__ void __launch_bounds__(TH, 1) k_sort_coop(const uint32_t* kin0, const
     }
     __syncthreads();
     // per digit: warp offsets (exclusive, in place) and the tile's count
-    uint32_t cnt[DPT], csum = 0;
+    uint32_t cnt = 0;
 #pragma unroll
-    for (int j = 0; j < DPT; j++) {
-      const int d = DPT * tid + j;
-      uint32_t c = 0;
-#pragma unroll
-      for (int w = 0; w < W; w++) {
-        unsigned short* h = reinterpret_cast<unsigned short*>(sm.whist[w]) + d;
-        const uint32_t x = *h;
-        *h = (unsigned short)c;
-        c += x;
-      }
-      cnt[j] = c;
-      csum += c;
+    for (int w = 0; w < W; w++) {
+      unsigned short* h = reinterpret_cast<unsigned short*>(sm.whist[w]) + tid;
+      const uint32_t x = *h;
+      *h = (unsigned short)cnt;
+      cnt += x;
     }
-    uint32_t* mine = counts + (size_t)tile * kRadix;
-#pragma unroll
-    for (int j = 0; j < DPT; j++) __stcg(mine + DPT * tid + j, cnt[j]);
+    // (a digit's count is at most TILE <= 8192)
+    __stcg(reinterpret_cast<unsigned short*>(counts) + (size_t)tile * kRadix + tid, (unsigned short)cnt);
     if (!grid_barrier(bar, ntiles, passed, err)) return;
-    uint32_t pre[DPT], tot[DPT], gsum = 0;
+    // Every block reads all tiles' counts (290 KB of 16-bit ones at 140 tiles,
+    // which bounds this phase): four digits a thread and every fourth tile,
+    // 8-byte loads, 16 in flight (each round waits one L2 round trip).  With a
+    // 32-bit count and one digit a thread: 1M-key sort 122 us against 112,
+    // 100,000-triangle build 92 against 83, 1M-triangle build 211 against 201.
+    constexpr int Q = kRadix / 4, GR = TH / Q, U = 16;
+    const int grp = tid / Q, q = tid % Q;
+    const uint2* rows = reinterpret_cast<const uint2*>(counts) + q;
+    auto sum = [&](int t0, int t1, uint4& o) {
+      for (int b = t0 + grp; b < t1; b += GR * U) {
+        uint2 x[U];
 #pragma unroll
-    for (int j = 0; j < DPT; j++) {
-      const uint32_t* col = counts + DPT * tid + j;
-      // 32 loads in flight per round (each round waits one L2 round trip)
-      constexpr int U = 32;
-      uint32_t acc = 0u, all = 0u;
-      for (int t0 = 0; t0 < ntiles; t0 += U) {
-        uint32_t x[U];
+        for (int u = 0; u < U; u++) x[u] = b + u * GR < t1 ? __ldcg(rows + (size_t)(b + u * GR) * Q) : make_uint2(0u, 0u);
 #pragma unroll
-        for (int u = 0; u < U; u++) x[u] = t0 + u < ntiles ? __ldcg(col + (size_t)(t0 + u) * kRadix) : 0u;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          all += x[u];
-          acc += t0 + u < tile ? x[u] : 0u;
+        for (int u = 0; u < U; u += 4) {  // four counts fit in 16 bits
+          const uint32_t lo = x[u].x + x[u + 1].x + x[u + 2].x + x[u + 3].x;
+          const uint32_t hi = x[u].y + x[u + 1].y + x[u + 2].y + x[u + 3].y;
+          o.x += lo & 0xffffu, o.y += lo >> 16, o.z += hi & 0xffffu, o.w += hi >> 16;
         }
       }
-      pre[j] = acc;
-      tot[j] = all;
-      gsum += all;
-    }
+    };
+    uint4 part = make_uint4(0u, 0u, 0u, 0u);
+    sum(0, tile, part);
+    reinterpret_cast<uint4*>(s_part[0][grp])[q] = part;
+    sum(tile, ntiles, part);
+    reinterpret_cast<uint4*>(s_part[1][grp])[q] = part;
+    __syncthreads();
+    uint32_t pre = 0, tot = 0;
+#pragma unroll
+    for (int k = 0; k < GR; k++) pre += s_part[0][k][tid], tot += s_part[1][k][tid];
     // digit starts (over all keys) and tile-local digit starts, in one scan
     uint32_t gpre, cpre;
-    block_excl_scan2<TH>(gsum, csum, sm.warp2, gpre, cpre);
-    {
-      uint32_t c = cpre, g = gpre;
-#pragma unroll
-      for (int j = 0; j < DPT; j++) {
-        const int d = DPT * tid + j;
-        sm.tstart[d] = c;
-        sm.gbase[d] = g + pre[j] - c;
-        c += cnt[j];
-        g += tot[j];
-      }
-    }
+    block_excl_scan2<TH>(tot, cnt, sm.warp2, gpre, cpre);
+    sm.tstart[tid] = cpre;
+    sm.gbase[tid] = gpre + pre - cpre;
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < IT; r++) {

@@ -32,3 +32,22 @@ def test_sort_shapes(cuda, n, bits, spread):
     if n <= crt.SORT_NOALLOC_MAX_PAIRS:
         crt.sort_pairs_noalloc(kd, vd, ko, vo, key_bits=bits)
         assert_equal(vo.cpu().numpy(), v[order], "values, no allocation")
+
+
+@pytest.mark.parametrize("n", [1025, 8192, 152 * 1024, 152 * 4096 + 1, 152 * 8192 - 5])
+@pytest.mark.parametrize("kind", ["equal", "two", "last tile"])
+def test_skewed_digits(cuda, n, kind):
+    """One digit holding whole tiles (the largest 16-bit counts), two digits, and a digit of the last tile alone."""
+    import torch
+    import crt
+    k = torch.full((n,), 0x2AA55AA5, dtype=torch.int32, device="cuda")
+    if kind == "two":
+        k[torch.arange(n, device="cuda") % 3 == 1] = 0x15455AA5
+    elif kind == "last tile":
+        k[-700:] = 0x00100400
+    v = torch.arange(n, dtype=torch.int32, device="cuda")
+    ko, vo = torch.empty_like(k), torch.empty_like(v)
+    crt.sort_pairs(k, v, ko, vo, key_bits=30)
+    ks, ix = torch.sort(k, stable=True)
+    assert torch.equal(ko, ks)
+    assert torch.equal(vo, v[ix])
