@@ -269,7 +269,9 @@ static __device__ __noinline__ bool box_exact(double ox, double oy, double oz, d
 // The bounds used take 64u for 46u and 8u for 6u,
 //   E_det = K |AB| |d| |AC|,  E_a = K |d| |AC| (|T| + |o| / 8),
 //   E_b = K |d| |AB| (|T| + |o| / 8),  K = 2^-18,
-// which covers the second order and the double computation's own error.  (With
+// which covers the second order and the double computation's own error; 1e-20
+// added to |T| + |o| / 8 covers products that underflow (a vertex within 1e-35 of
+// the ray's start).  (With
 // K = 2^-16 and |o| in place of |o| / 8, four to eight times the candidates were
 // left to exact tests: large frame 13.6 ms against 10.8, recursive 13.8 against
 // 12.4, 500k any-hit rays 435 us against 386.)
@@ -301,7 +303,7 @@ __device__ __forceinline__ bool tri_reject_sure(const RayC& r, float4 a, float4 
   const float nT = fmaxf(fmaxf(fabsf(Tx), fabsf(Ty)), fabsf(Tz));
   const float nd = fmaxf(fmaxf(fabsf(r.fdx), fabsf(r.fdy)), fabsf(r.fdz));
   const float K = 3.814697265625e-06f;  // 2^-18
-  const float ot = __fadd_ru(nT, 0.125f * r.omax);
+  const float ot = __fadd_ru(nT, __fmaf_ru(0.125f, r.omax, 1e-20f));
   const float Ed = __fmul_ru(__fmul_ru(__fmul_ru(K, nAB), nd), nAC);
   const float Ea = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAC), ot);
   const float Eb = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAB), ot);
@@ -348,7 +350,7 @@ __device__ __forceinline__ TriClass tri_class(const RayC& r, float4 a, float4 b,
   const float nT = fmaxf(fmaxf(fabsf(Tx), fabsf(Ty)), fabsf(Tz));
   const float nd = fmaxf(fmaxf(fabsf(r.fdx), fabsf(r.fdy)), fabsf(r.fdz));
   const float K = 3.814697265625e-06f;  // 2^-18
-  const float ot = __fadd_ru(nT, 0.125f * r.omax);
+  const float ot = __fadd_ru(nT, __fmaf_ru(0.125f, r.omax, 1e-20f));
   const float Ed = __fmul_ru(__fmul_ru(__fmul_ru(K, nAB), nd), nAC);
   const float Ea = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAC), ot);
   const float Eb = __fmul_ru(__fmul_ru(__fmul_ru(K, nd), nAB), ot);
@@ -631,7 +633,8 @@ __device__ __forceinline__ void cswap(float& ta, int& ca, float& tb, int& cb) {
 // together.  On soups, whose rays leave their warp, that ends most of the waiting
 // (100,000 triangles 640x480x1: 859 -> 706 us; the 24-mesh batch 21.6 -> 15.0
 // ms); on the large sphere, whose rays stay together, little changes (13.78 ->
-// 13.68 ms).  The recursive kernel is 7% slower with it and leaves it out.
+// 13.68 ms).  The recursive kernel gains nothing from it (11.24 against 11.23
+// ms at depth 3) and leaves it out.
 // ANY: returns 1 when the first hit in DFS order lies between the ray's start
 // and `dist` along it (a shadow ray, Light.cu:14-16: t < dist and not t <
 // RAY_EPSILON), with h.id set; 0 otherwise.

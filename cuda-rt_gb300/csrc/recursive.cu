@@ -33,9 +33,9 @@ namespace {
 
 // The most lanes a pixel's samples take when there are secondary rays (fewer
 // when spp is smaller): on the depth-3 mirror/glass frame (1280x720, 4 spp)
-// 2 lanes took 16.0 ms, 4 lanes 18.3 ms (more walks start from wrong guesses)
-// and 1 lane 19.0 ms.  Without secondary rays (depth 0) one lane per pixel
-// is fastest (3.3 against 3.5 ms): there is no tree to overlap.  Small images
+// 2 lanes took 12.1 ms, 4 lanes 13.0 ms (more walks start from wrong guesses);
+// 1 lane was 19% slower than 2.  Without secondary rays (depth 0) one lane per
+// pixel is fastest (by 6%): there is no tree to overlap.  Small images
 // take up to four (spread_pixels).
 constexpr int kRecLanesPerPixel = 2;
 

@@ -136,3 +136,30 @@ def test_flat_boxes(cuda, axis, offset):
         assert_equal(gi, oi, f"ids any={any_hit}")
         assert_equal(gt, ot, f"t any={any_hit}")
     g.check()
+
+
+def test_underflowing_products(cuda):
+    """Rays that start within 1e-20 to 1e-38 of a vertex near the origin: the filters' products underflow."""
+    import crt
+    from crt import data
+    from oracle.oracle import OracleScene
+    rng = np.random.default_rng(13)
+    n = 60
+    v = rng.normal(size=(n, 3, 3))
+    v[:, 0] = rng.normal(size=(n, 3)) * 10.0 ** rng.uniform(-38, -20, (n, 1))  # every triangle has a vertex there
+    v = v.reshape(-1, 3).astype(np.float32)
+    idx = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    nrm = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (3 * n, 1))
+    m = data.Mesh(v, idx, nrm, idx.copy(), np.zeros(n, np.int32), data.lambert_material()[None])
+    g, o = crt.Scene(m), OracleScene(m)
+    count = 4_000
+    start = rng.normal(size=(count, 3)) * 10.0 ** rng.uniform(-38, -20, (count, 1))
+    d = rng.normal(size=(count, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.hstack([start - d * np.where(rng.random((count, 1)) < 0.5, 0.0, 1.0), d])
+    for any_hit in (False, True):
+        gi, gt = g.trace(rays, any_hit=any_hit)
+        oi, ot, _ = o.trace(rays, any_hit=any_hit)
+        assert_equal(gi, oi, f"ids any={any_hit}")
+        assert_equal(gt, ot, f"t any={any_hit}")
+    g.check()
