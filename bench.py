@@ -50,10 +50,10 @@ W, H, SPP = 1920, 1080, 16
 # lens-table lookups (two random loads per sample, each filling whole L2
 # lines) and the threads' local memory (traversal stacks and register spills
 # of 175,104 resident threads).  Re-captured whenever those kernels change.
-RENDER_DRAM_BYTES = 11_957_783_808
-BUILD_DRAM_BYTES = 227_666_176
-BUILD_L2_BYTES = 869_048_800
-TRAFFIC_SOURCE = "ncu 2025.3 single-pass captures, GB300, 2026-12-04"
+RENDER_DRAM_BYTES = 6_044_910_000
+BUILD_DRAM_BYTES = 144_885_000
+BUILD_L2_BYTES = 679_664_000
+TRAFFIC_SOURCE = "ncu 2025.3 single-pass captures, GB300, 2026-12-05"
 
 
 def build_launches(n):
@@ -209,8 +209,8 @@ def run_crt(args, dist, rank, ws):
     ms_step = t_total / args.steps * 1e3
     hbm, peak_kind = peaks()
     # render roofline (the dominant kernel): the bytes the traversal fetches,
-    # 128 B per visited four-wide node + 48 B per tested leaf triangle, per launch
-    alg_bytes = nodes_visited * 128 + tris_tested * 48
+    # 64 B per visited four-wide node + 48 B per tested leaf triangle, per launch
+    alg_bytes = nodes_visited * 64 + tris_tested * 48
     render_s = t_render / args.steps
     achieved = alg_bytes / render_s / 1e9
     build_s = t_build / args.steps
