@@ -58,12 +58,12 @@ TRAFFIC_SOURCE = "ncu 2025.3 single-pass captures, GB300, 2026-12-05"
 
 def build_launches(n):
     """Kernel launches of one crt_bvh_build of n triangles (build.cu): init,
-    bounds, Morton, the sort (one cooperative launch from 16,384 triangles
+    bounds, Morton, the sort (one cooperative launch from 32,768 triangles
     up to 152 tiles of 8192, else three passes), split search, refit and,
     above one 512-leaf refit block, the spanning-node refit."""
     if n <= 0:
         return 0
-    sort = 1 if 2 * 8192 <= n <= 152 * 8192 else 3
+    sort = 1 if 4 * 8192 <= n <= 152 * 8192 else 3
     return 3 + sort + (1 if n >= 2 else 0) + 1 + (1 if n > 512 else 0)
 
 

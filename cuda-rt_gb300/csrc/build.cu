@@ -798,11 +798,12 @@ static void refit(const MeshBufs& m, const BuildBufs& b, cudaStream_t st) {
 // 8 and the shorter barrier make it 211.5 us from 216.5.)  The build takes it
 // from kCoopBuildMin keys on: below, three look-back passes launched as
 // programmatic dependents cost less than the cooperative launch (2000
-// triangles 43 against 54 us, 16,000 58 against 61).  The standalone sort,
+// triangles 43 against 54 us, 16,000 57.7 against 61.6, 19,220 58.1 against 60.9; 40,000
+// 74.8 against 73.9, 100,000 101.6 against 82.3).  The standalone sort,
 // which would also need a histogram pass, takes it from 1025 keys on (3000
 // 16-bit keys 55 against 64 us, 20,000 32-bit ones 73 against 78, 1,000,003
 // 131 against 137).
-constexpr int kCoopBuildMin = 2 * kSortTileL, kCoopSortMin = kSortThreadsL + 1;
+constexpr int kCoopBuildMin = 4 * kSortTileL, kCoopSortMin = kSortThreadsL + 1;
 using CoopSort = void (*)(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, int, int,
                           uint32_t*, unsigned*, int*);
 constexpr int kCoopItems[] = {1, 2, 4, 7, 8};

@@ -51,3 +51,15 @@ def test_skewed_digits(cuda, n, kind):
     ks, ix = torch.sort(k, stable=True)
     assert torch.equal(ko, ks)
     assert torch.equal(vo, v[ix])
+
+
+@pytest.mark.parametrize("n", [16384, 32767, 32768, 32769])
+def test_builds_beside_the_cooperative_sort(cuda, n):
+    """Builds on both sides of the size from which their sort is one cooperative launch."""
+    import crt
+    from crt import data
+    from oracle.oracle import OracleScene
+    m = data.soup(n, seed=n)
+    ge, oe = crt.Scene(m).export(), OracleScene(m).export()
+    for k in ("codes", "ids", "nodes", "node_boxes"):
+        assert_equal(ge[k], oe[k], k)
