@@ -183,12 +183,14 @@ cudaError_t launch_trace(const DScene& S, const double* rays, int64_t n, bool an
   else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_trace<false>, 128, 0);
   if (bps <= 0) bps = 1;
-  // few rays are spread over more warps: a walk's latency, not the lanes,
-  // then bounds the call (4096 rays: 248 us with 32 to a warp, 166 us with 2,
-  // both with the 100 us rebuild before them)
+  // few rays are spread over more warps, down to one ray each: a walk's latency,
+  // not the lanes, then bounds the call (4096 view rays against 19,220
+  // triangles, with the rebuild before them: 32 to a warp 248 us, 4 144, 2 129, 1
+  // 127; without it 2000 incoherent rays against 100,000 triangles: 4 214 us, 2
+  // 171, 1 133; 8000: 234, 216, 188)
   const int64_t warps = (int64_t)num_sms() * bps * 4;
   int per = 32;
-  while (per > 2 && (n + per - 1) / per < warps) per /= 2;
+  while (per > 1 && (n + per - 1) / per < warps) per /= 2;
   const int64_t need = ((n + per - 1) / per + 3) / 4;
   const int grid = (int)(need < (int64_t)num_sms() * bps ? need : (int64_t)num_sms() * bps);
   if (any)
