@@ -212,6 +212,11 @@ static bool slot_contains(const WNode& w, int slot, const float box[6]) {
   return true;
 }
 
+// The device's fminf and fmaxf: -0 orders below +0 (the host's std::fmin and
+// std::fmax may return either zero, by the operands' order).
+static float min_z(float a, float b) { return a == b ? (std::signbit(a) ? a : b) : std::fmin(a, b); }
+static float max_z(float a, float b) { return a == b ? (std::signbit(a) ? b : a) : std::fmax(a, b); }
+
 bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* leaves, const float* root_box,
                  int* nodes3, float* boxes) {
   const int ni = n - 1;
@@ -230,8 +235,8 @@ bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* 
     int x = ni + k;
     float* bx = boxes + 6 * (size_t)x;
     for (int c = 0; c < 3; c++) {
-      bx[c] = std::fmin(v[2][c], std::fmin(v[0][c], v[1][c]));
-      bx[3 + c] = std::fmax(v[2][c], std::fmax(v[0][c], v[1][c]));
+      bx[c] = min_z(v[2][c], min_z(v[0][c], v[1][c]));
+      bx[3 + c] = max_z(v[2][c], max_z(v[0][c], v[1][c]));
     }
     while (x != 0 && n > 1) {
       const int p = nodes3[3 * x];
@@ -239,7 +244,7 @@ bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* 
       if (seen[p] > 2) return false;
       const float *l = boxes + 6 * (size_t)nodes3[3 * p + 1], *r = boxes + 6 * (size_t)nodes3[3 * p + 2];
       float* o = boxes + 6 * (size_t)p;
-      for (int c = 0; c < 3; c++) o[c] = std::fmin(l[c], r[c]), o[3 + c] = std::fmax(l[3 + c], r[3 + c]);
+      for (int c = 0; c < 3; c++) o[c] = min_z(l[c], r[c]), o[3 + c] = max_z(l[3 + c], r[3 + c]);
       x = p;
     }
   }
