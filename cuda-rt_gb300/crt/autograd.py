@@ -13,6 +13,8 @@ C through include/crt.h.
 """
 from __future__ import annotations
 
+import contextlib
+
 import numpy as np
 import torch
 
@@ -54,12 +56,27 @@ class Renderer:
         self.camera, self.light = camera, light
         self.W, self.H, self.spp = width, height, spp
 
+    @contextlib.contextmanager
+    def _stream(self):
+        """torch's current stream, for the library's calls as well: their inputs, outputs and temporaries are in order
+        with torch's operations, and nothing waits on the host.  The scene and its material table are shared by all
+        calls, whichever stream they come from, and by callers of the scene itself: a stream other than the default one
+        (the library's own) takes its turn on that one."""
+        stream, default = torch.cuda.current_stream(), torch.cuda.default_stream()
+        if stream != default:
+            stream.wait_stream(default)
+        try:
+            yield stream
+        finally:
+            if stream != default:
+                default.wait_stream(stream)
+
     def set_inputs(self, verts, light_pos, albedo):
-        self.scene.set_vertices(verts.detach().contiguous(), rebuild=True)
-        self.mats[:, 3:6] = albedo.detach().to(self.mats.device, torch.float64)
+        with self._stream() as stream:
+            self.scene.set_vertices(verts.detach().contiguous(), rebuild=True, stream=stream)
+            self.mats[:, 3:6] = albedo.detach().to(self.mats.device, torch.float64)
+            self.scene.set_materials(self.mats, stream=stream)
         lp = tuple(float(x) for x in light_pos.detach().cpu().numpy())
-        torch.cuda.current_stream().synchronize()  # (the library works on the default stream)
-        self.scene.set_materials(self.mats)
         self.cur_light = Light(position=lp, color=self.light.color, radius=self.light.radius,
                                constant_term=self.light.constant_term, linear_term=self.light.linear_term,
                                quadratic_term=self.light.quadratic_term)
@@ -68,7 +85,9 @@ class Renderer:
         n = self.W * self.H
         img = torch.empty((n, 3), dtype=torch.float64, device="cuda")
         depth = torch.empty(n, dtype=torch.float64, device="cuda")
-        self.scene.render(self.camera, self.cur_light, self.W, self.H, self.spp, out={"rgb_f64": img, "depth": depth})
+        with self._stream() as stream:
+            self.scene.render(self.camera, self.cur_light, self.W, self.H, self.spp,
+                              out={"rgb_f64": img, "depth": depth}, stream=stream)
         return img, depth
 
     def adjoint(self, grad_img, grad_depth=None):
@@ -77,8 +96,9 @@ class Renderer:
                    light=torch.zeros(3, dtype=torch.float64, device=dev),
                    kd=torch.zeros((self.scene.nmat, 3), dtype=torch.float64, device=dev))
         gd = None if grad_depth is None else grad_depth.contiguous().to(torch.float64)
-        self.scene.adjoint(self.camera, self.cur_light, self.W, self.H, self.spp,
-                           grad_img.contiguous().to(torch.float64), gd, out=out)
+        with self._stream() as stream:
+            self.scene.adjoint(self.camera, self.cur_light, self.W, self.H, self.spp,
+                               grad_img.contiguous().to(torch.float64), gd, out=out, stream=stream)
         return out
 
 
