@@ -122,7 +122,7 @@ __device__ __forceinline__ double norm_exact(D3 a) {
 struct RayC {
   double ox, oy, oz, dx, dy, dz;
   float fox, foy, foz, fdx, fdy, fdz;  // origin, direction rounded to float
-  float omax;            // max |origin| component (float, rounded up)
+  float omax;            // max |origin| component (float, rounded up); +inf: no triangle bounds (see ray_setup)
   float ax, ay, az;      // 1/d in float; 0 on a "free" axis
   float lx, ly, lz;      // RD(c - m), c = RN(-o_f * a_f)
   float hx, hy, hz;      // RU(c + m)
@@ -163,8 +163,13 @@ __device__ __forceinline__ void ray_setup(RayC& r, double ox, double oy, double 
   r.fdx = fd[0], r.fdy = fd[1], r.fdz = fd[2];
   // |o| rounded up: float rounding of o is at most a relative 2^-24
   const float omax = __fmul_ru(fmaxf(fmaxf(fabsf(fo[0]), fabsf(fo[1])), fabsf(fo[2])), 1.0000002f);
-  r.omax = omax;
   const float reach = __fmul_ru(1.7320509f, __fadd_ru(omax, B));
+  // The triangle filters' determinant and numerators, at most 24 |d| B (B + |o|)
+  // in max-norms, must be finite: with one product overflowed and the others not,
+  // a sum has the wrong sign.  Where they might not be, the infinite omax makes
+  // their bounds infinite, and the exact test decides.
+  const float nd = fmaxf(fmaxf(fabsf(fd[0]), fabsf(fd[1])), fabsf(fd[2]));
+  r.omax = __fmul_ru(__fmul_ru(nd, B), reach) <= 1e37f ? omax : __int_as_float(0x7f800000);
   const float D2 = __fmul_ru(D, D);
   // 2^-29 / 1e-8 and 2^-30 / 1e-8, rounded up
   const float eps = __fmul_ru(__fmul_ru(0.18626452f, D2), __fadd_ru(reach, D));
