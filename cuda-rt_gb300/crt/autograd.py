@@ -72,11 +72,12 @@ class Renderer:
                 default.wait_stream(stream)
 
     def set_inputs(self, verts, light_pos, albedo):
+        # (read before anything is queued: the wait for the copy then covers only earlier work)
+        lp = tuple(float(x) for x in light_pos.detach().cpu().numpy())
         with self._stream() as stream:
             self.scene.set_vertices(verts.detach().contiguous(), rebuild=True, stream=stream)
             self.mats[:, 3:6] = albedo.detach().to(self.mats.device, torch.float64)
             self.scene.set_materials(self.mats, stream=stream)
-        lp = tuple(float(x) for x in light_pos.detach().cpu().numpy())
         self.cur_light = Light(position=lp, color=self.light.color, radius=self.light.radius,
                                constant_term=self.light.constant_term, linear_term=self.light.linear_term,
                                quadratic_term=self.light.quadratic_term)
