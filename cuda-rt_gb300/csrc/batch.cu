@@ -281,7 +281,7 @@ crt_status crt_batch_create(const crt_mesh_desc* meshes, const crt_batch_view* v
   std::vector<size_t> off(K);
   size_t total = 0;
   for (int i = 0; i < K; i++) off[i] = total, total += al(sz[i]);
-  cudaError_t e = cudaMalloc(&b->block, total);
+  cudaError_t e = device_alloc(reinterpret_cast<void**>(&b->block), total);
   if (e != cudaSuccess) {
     delete b;
     return cuda_fail(e, "cudaMalloc");

@@ -24,6 +24,8 @@ struct crt_scene {
   unsigned* counter = nullptr;
   void* block = nullptr;  // one allocation backing the build arrays
   size_t block_bytes = 0;
+  int pool_dev = -1;  // the scratch pool's device and context that count this scene
+  unsigned long long pool_ctx = 0;
 };
 
 namespace {
@@ -81,40 +83,72 @@ DScene dscene(const crt_scene* s) {
 // one per device, that keeps up to kScratchKept bytes between calls.  (The
 // device's default pool keeps nothing: every call that allocates and then
 // synchronises maps its memory anew.)  Allocation stays stream-ordered, so
-// calls on several streams and threads never share a block.  Destroying a
-// scene gives the kept memory back.  While a stream is captured, on another
-// device's stream, or when the pool cannot serve, the default pool is used.
+// calls on several streams and threads never share a block.  The kept memory
+// goes back when the last scene of the device is destroyed, on request while
+// there is none (crt_scene_destroy(NULL)), and when an allocation of the
+// library would fail without it.  While a stream is captured, on another
+// device's stream, in a context other than the device's primary one (its id
+// would come and go in the device's slot), or when the pool cannot serve, the
+// default pool is used.
 constexpr int kMaxDevices = 64;
 constexpr uint64_t kScratchKept = (uint64_t)256 << 20;
 struct ScratchPool {
-  unsigned long long ctx_id = 0;  // the CUDA context the pool was made in
-  cudaMemPool_t pool = nullptr;
+  unsigned long long ctx_id = 0;  // the primary context the pool was made in; cudaDeviceReset ends both
+  cudaMemPool_t pool = nullptr;   // made on first use
+  int64_t scenes = 0;             // alive in that context
 };
 std::mutex g_pool_mu;
 ScratchPool g_pool[kMaxDevices];
 
-// The current context's pool, made on first use (make), or NULL.
-cudaMemPool_t scratch_pool(bool make) {
+// The current device's slot (the caller holds g_pool_mu), or NULL.
+ScratchPool* scratch_slot() {
   int dev = 0;
   unsigned long long id = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices || !current_context_id(&id)) return nullptr;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices || !primary_context_id(&id)) return nullptr;
+  if (g_pool[dev].ctx_id != id) g_pool[dev] = ScratchPool{id, nullptr, 0};
+  return &g_pool[dev];
+}
+
+cudaMemPool_t scratch_pool() {
   std::lock_guard<std::mutex> lock(g_pool_mu);
-  ScratchPool& p = g_pool[dev];
-  if (p.pool && p.ctx_id == id) return p.pool;
-  p.pool = nullptr;
-  if (!make) return nullptr;
+  ScratchPool* p = scratch_slot();
+  if (!p || p->pool) return p ? p->pool : nullptr;
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = dev;
+  props.location.id = (int)(p - g_pool);
   uint64_t kept = kScratchKept;
-  if (cudaMemPoolCreate(&p.pool, &props) != cudaSuccess ||
-      cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) {
-    cudaGetLastError();
-    p.pool = nullptr;
+  cudaMemPool_t made = nullptr;
+  if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
+    if (cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &kept) == cudaSuccess)
+      p->pool = made;
+    else
+      cudaMemPoolDestroy(made);
   }
-  p.ctx_id = id;
-  return p.pool;
+  if (!p->pool) cudaGetLastError();
+  return p->pool;
+}
+
+// Gives the current device's kept memory back, if it has any (idle: only when no scene is alive).
+bool scratch_trim(bool idle) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ScratchPool* p = scratch_slot();
+  return p && p->pool && !(idle && p->scenes > 0) && cudaMemPoolTrimTo(p->pool, 0) == cudaSuccess;
+}
+
+void scratch_scene_born(crt_scene* s) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ScratchPool* p = scratch_slot();
+  if (!p) return;
+  s->pool_dev = (int)(p - g_pool), s->pool_ctx = p->ctx_id;
+  p->scenes++;
+}
+
+void scratch_scene_gone(const crt_scene* s) {
+  if (s->pool_dev < 0) return;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ScratchPool& p = g_pool[s->pool_dev];
+  if (p.ctx_id == s->pool_ctx && --p.scenes == 0 && p.pool) cudaMemPoolTrimTo(p.pool, 0);
 }
 
 cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t st) {
@@ -124,15 +158,12 @@ cudaError_t scratch_alloc(void** out, size_t bytes, cudaStream_t st) {
                      (st && (cudaGetDevice(&dev) != cudaSuccess || cudaStreamGetDevice(st, &sdev) != cudaSuccess ||
                              dev != sdev));
   if (!plain)
-    if (cudaMemPool_t p = scratch_pool(true)) {
+    if (cudaMemPool_t p = scratch_pool()) {
       if (cudaMallocFromPoolAsync(out, bytes, p, st) == cudaSuccess) return cudaSuccess;
       cudaGetLastError();
+      scratch_trim(false);
     }
   return cudaMallocAsync(out, bytes, st);
-}
-
-void scratch_trim() {
-  if (cudaMemPool_t p = scratch_pool(false)) cudaMemPoolTrimTo(p, 0);
 }
 
 // A device view of a caller buffer: the buffer itself when it is device
@@ -197,6 +228,15 @@ void free_scene(crt_scene* s) {
 }  // namespace
 
 namespace crt {
+cudaError_t device_alloc(void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaErrorMemoryAllocation && scratch_trim(false)) {
+    cudaGetLastError();
+    e = cudaMalloc(out, bytes);
+  }
+  return e;
+}
+
 // Lets entry points in other translation units record their error message.
 void set_last_error(const char* msg) { g_err = msg; }
 
@@ -327,7 +367,7 @@ static crt_status create_scene(const crt_mesh_desc* d, void* stream, bool borrow
   };
   cudaError_t e;
 #define ALLOC(ptr, bytes)                                                 \
-  if ((bytes) > 0 && (e = cudaMalloc(&(ptr), (bytes))) != cudaSuccess) \
+  if ((bytes) > 0 && (e = device_alloc(reinterpret_cast<void**>(&(ptr)), (bytes))) != cudaSuccess) \
     return bail(e, "cudaMalloc");
   s->borrowed = borrow;
   if (borrow) {
@@ -426,6 +466,7 @@ static crt_status create_scene(const crt_mesh_desc* d, void* stream, bool borrow
     delete s;
     return fail(r, msg);
   }
+  scratch_scene_born(s);
   *out = s;
   return CRT_OK;
 }
@@ -439,11 +480,14 @@ crt_status crt_scene_create_borrowed(const crt_mesh_desc* d, void* stream, crt_s
 }
 
 crt_status crt_scene_destroy(crt_scene* s) {
-  if (!s) return CRT_OK;
+  if (!s) {
+    scratch_trim(true);
+    return CRT_OK;
+  }
   cudaDeviceSynchronize();
   free_scene(s);
+  scratch_scene_gone(s);
   delete s;
-  scratch_trim();
   return CRT_OK;
 }
 

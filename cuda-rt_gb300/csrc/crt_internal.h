@@ -89,6 +89,11 @@ int num_sms();
 // sort_noalloc.cu: the id of the current CUDA context, unique for the life of
 // the process (a context that cudaDeviceReset destroyed never comes back).
 bool current_context_id(unsigned long long* id);
+// The same, false unless the current context is its device's primary one.
+bool primary_context_id(unsigned long long* id);
+
+// capi.cu: cudaMalloc, tried again without the scratch pool's kept memory when there is not enough.
+cudaError_t device_alloc(void** out, size_t bytes);
 
 // capi.cu: the reference's nodes (parent, left, right; leaves get their parent
 // only) and exact boxes of a downloaded tree, for the exports: the topology

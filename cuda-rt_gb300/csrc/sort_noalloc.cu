@@ -41,6 +41,10 @@ namespace {
 // cudaDeviceReset has since destroyed is never reused.
 typedef int (*CtxGetCurrentFn)(void** ctx);
 typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
+typedef int (*CtxGetDeviceFn)(int* dev);
+typedef int (*PrimaryStateFn)(int dev, unsigned* flags, int* active);
+typedef int (*PrimaryRetainFn)(void** ctx, int dev);
+typedef int (*PrimaryReleaseFn)(int dev);
 void* driver_fn(const char* name) {
   void* f = nullptr;
   cudaDriverEntryPointQueryResult q;
@@ -59,6 +63,23 @@ bool current_context_id(unsigned long long* id) {
   static CtxGetIdFn get_id = reinterpret_cast<CtxGetIdFn>(driver_fn("cuCtxGetId"));
   void* ctx = nullptr;
   return get_current && get_id && get_current(&ctx) == 0 && ctx && get_id(ctx, id) == 0;
+}
+
+bool primary_context_id(unsigned long long* id) {
+  static CtxGetCurrentFn get_current = reinterpret_cast<CtxGetCurrentFn>(driver_fn("cuCtxGetCurrent"));
+  static CtxGetDeviceFn get_device = reinterpret_cast<CtxGetDeviceFn>(driver_fn("cuCtxGetDevice"));
+  static PrimaryStateFn state = reinterpret_cast<PrimaryStateFn>(driver_fn("cuDevicePrimaryCtxGetState"));
+  static PrimaryRetainFn retain = reinterpret_cast<PrimaryRetainFn>(driver_fn("cuDevicePrimaryCtxRetain"));
+  static PrimaryReleaseFn release = reinterpret_cast<PrimaryReleaseFn>(driver_fn("cuDevicePrimaryCtxRelease"));
+  if (!get_current || !get_device || !state || !retain || !release) return false;
+  void *ctx = nullptr, *primary = nullptr;
+  int dev = 0, active = 0;
+  unsigned flags = 0;
+  if (get_current(&ctx) != 0 || !ctx || get_device(&dev) != 0 || state(dev, &flags, &active) != 0 || !active ||
+      retain(&primary, dev) != 0)
+    return false;
+  release(dev);  // (held by others: it is the current context)
+  return primary == ctx && current_context_id(id);
 }
 }  // namespace crt
 

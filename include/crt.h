@@ -133,6 +133,11 @@ crt_status crt_scene_create(const crt_mesh_desc* mesh, void* stream, crt_scene**
  * crt_scene_set_vertices(scene, NULL, rebuild, stream) refits or rebuilds
  * from them (a non-NULL array is refused, as is crt_scene_set_materials). */
 crt_status crt_scene_create_borrowed(const crt_mesh_desc* mesh, void* stream, crt_scene** out);
+/* Frees the scene.  Calls that need scratch or stage host arrays (renders,
+ * traces, the adjoint, the sort, the build stages) keep up to 256 MB of device
+ * memory per device between calls; destroying the device's last scene gives it
+ * back, and so does crt_scene_destroy(NULL) with that device current while no
+ * scene is alive (a program that only sorts). */
 crt_status crt_scene_destroy(crt_scene* scene);
 
 /* New vertex positions for the same triangles (num_vertices * 3 floats),
@@ -265,8 +270,9 @@ crt_status crt_refit(const float* vertices, int32_t num_vertices, const int32_t*
  * vals_in may be NULL: values are then 0..n-1.  Device pointers of the
  * current device.  It does not sort in place: an input array that overlaps
  * an output array, or two overlapping outputs, are refused with
- * CRT_INVALID_ARG.  Scratch is allocated per call (cudaMallocAsync); the call
- * synchronises `stream` and reports a look-back timeout as CRT_TIMEOUT. */
+ * CRT_INVALID_ARG.  Scratch comes from the memory kept between calls (see
+ * crt_scene_destroy) or cudaMallocAsync; the call synchronises `stream` and
+ * reports a look-back timeout as CRT_TIMEOUT. */
 crt_status crt_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
                           int32_t n, int32_t key_bits, void* stream);
 
