@@ -811,7 +811,7 @@ constexpr CoopSort kCoopSort[] = {k_sort_coop<kSortThreadsL, 1>, k_sort_coop<kSo
                                   k_sort_coop<kSortThreadsL, 4>, k_sort_coop<kSortThreadsL, 7>,
                                   k_sort_coop<kSortThreadsL, 8>};
 constexpr int kCoopShapes = sizeof(kCoopItems) / sizeof(kCoopItems[0]);
-static int coop_shape(int n, int least) {
+static int coop_shape(int n, int least, cudaStream_t st) {
   static int capacity = -1;  // one block per SM at least, or none
   if (capacity < 0) {
     int bps = 0;
@@ -821,7 +821,9 @@ static int coop_shape(int n, int least) {
     }
     capacity = bps > 0 ? num_sms() : 0;
   }
-  if (n < least) return -1;
+  // (a green context may hold fewer SMs than the device has, and its stream then
+  // could not run the tiles' blocks all at once: the look-back passes need no such thing)
+  if (n < least || in_green_context(st)) return -1;
   for (int i = 0; i < kCoopShapes; i++)
     if (((int64_t)n + kSortThreadsL * kCoopItems[i] - 1) / (kSortThreadsL * kCoopItems[i]) <= capacity) return i;
   return -1;
@@ -847,7 +849,7 @@ cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st)
   if (n <= 0) return cudaSuccess;
   const int passes = 3;
   const int tiles = sort_tiles(n);
-  const int shape = coop_shape(n, kCoopBuildMin);
+  const int shape = coop_shape(n, kCoopBuildMin, st);
   const bool coop = shape >= 0;
   k_build_init<<<1, 1024, 0, st>>>(b.g, b.hist, passes * kRadix, b.gbox, (int)span_groups(n));
   const int sms = num_sms();
@@ -865,8 +867,9 @@ cudaError_t launch_build(const MeshBufs& m, const BuildBufs& b, cudaStream_t st)
   if (coop) {
     // (counts: ntiles rows of the look-back status; barrier word:
     // tile_counter[0], zeroed by k_build_init)
-    launch_coop_sort(shape, b.keys_a, nullptr, b.keys_b, b.vals_b, b.keys_a, b.vals_a, n, passes, b.status,
-                     &b.g->tile_counter[0], &b.g->err, st);
+    const cudaError_t e = launch_coop_sort(shape, b.keys_a, nullptr, b.keys_b, b.vals_b, b.keys_a, b.vals_a, n,
+                                           passes, b.status, &b.g->tile_counter[0], &b.g->err, st);
+    if (e != cudaSuccess) return e;
   } else {
     const uint32_t* kin = b.keys_a;
     const uint32_t* vin = nullptr;
@@ -1071,7 +1074,7 @@ cudaError_t launch_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t
   uint32_t* status = hist + passes * kRadix;
   unsigned* counters = status + (size_t)passes * tiles * kRadix;
   // (one pass leaves room for half the rows that 1024-key tiles need)
-  const int shape = passes >= 2 ? coop_shape(n, kCoopSortMin) : -1;
+  const int shape = passes >= 2 ? coop_shape(n, kCoopSortMin, st) : -1;
   if (shape >= 0) {
     const cudaError_t e = cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;

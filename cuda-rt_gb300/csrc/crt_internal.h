@@ -91,6 +91,8 @@ int num_sms();
 bool current_context_id(unsigned long long* id);
 // The same, false unless the current context is its device's primary one.
 bool primary_context_id(unsigned long long* id);
+// Whether st's work runs in a green context, which may hold a part of the SMs only.
+bool in_green_context(cudaStream_t st);
 
 // capi.cu: cudaMalloc, tried again without the scratch pool's kept memory when there is not enough.
 cudaError_t device_alloc(void** out, size_t bytes);

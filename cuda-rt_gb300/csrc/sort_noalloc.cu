@@ -45,10 +45,11 @@ typedef int (*CtxGetDeviceFn)(int* dev);
 typedef int (*PrimaryStateFn)(int dev, unsigned* flags, int* active);
 typedef int (*PrimaryRetainFn)(void** ctx, int dev);
 typedef int (*PrimaryReleaseFn)(int dev);
-void* driver_fn(const char* name) {
+typedef int (*StreamGetGreenCtxFn)(cudaStream_t stream, void** ctx);
+void* driver_fn(const char* name, unsigned version = 12000) {
   void* f = nullptr;
   cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+  if (cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &q) != cudaSuccess ||
       q != cudaDriverEntryPointSuccess) {
     cudaGetLastError();
     return nullptr;
@@ -80,6 +81,14 @@ bool primary_context_id(unsigned long long* id) {
     return false;
   release(dev);  // (held by others: it is the current context)
   return primary == ctx && current_context_id(id);
+}
+bool in_green_context(cudaStream_t st) {
+  static StreamGetGreenCtxFn get_green =
+      reinterpret_cast<StreamGetGreenCtxFn>(driver_fn("cuStreamGetGreenCtx", 12040));
+  // (the default streams' handles stand for a stream of the current context)
+  void* green = nullptr;
+  return get_green && get_green(st == cudaStreamLegacy || st == cudaStreamPerThread ? nullptr : st, &green) == 0 &&
+         green;
 }
 }  // namespace crt
 
