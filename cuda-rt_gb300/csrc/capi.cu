@@ -269,6 +269,7 @@ bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* 
   }
   // boxes: the leaves' from their triangles, then unions upwards, the second child to arrive taking its parent's
   std::vector<char> seen(ni > 0 ? ni : 1, 0);
+  bool numbers = true;  // (a leaf whose corners are all NaN on an axis has no box there; the scene's check reports it)
   for (int k = 0; k < n; k++) {
     const LeafTri& t = leaves[k];
     const float v[3][3] = {{t.v0.x, t.v0.y, t.v0.z}, {t.v1.x, t.v1.y, t.v1.z}, {t.v2.x, t.v2.y, t.v2.z}};
@@ -277,6 +278,7 @@ bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* 
     for (int c = 0; c < 3; c++) {
       bx[c] = min_z(v[2][c], min_z(v[0][c], v[1][c]));
       bx[3 + c] = max_z(v[2][c], max_z(v[0][c], v[1][c]));
+      numbers = numbers && bx[c] == bx[c];
     }
     while (x != 0 && n > 1) {
       const int p = nodes3[3 * x];
@@ -288,9 +290,9 @@ bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* 
       x = p;
     }
   }
-  if (std::memcmp(boxes, root_box, 6 * sizeof(float)) != 0 && n > 1) return false;
+  if (numbers && n > 1 && std::memcmp(boxes, root_box, 6 * sizeof(float)) != 0) return false;
   // every slot of every wide node names the right node and contains its box (where the traversal looks at boxes)
-  bool filtered = true;
+  bool filtered = numbers;
   for (int c = 0; c < 6; c++) filtered = filtered && std::fabs(root_box[c]) <= kMaxFilterCoord;
   auto code_of = [&](int x) { return x < ni ? x : ~(x - ni); };
   for (int i = 0; i < ni; i++)
