@@ -240,14 +240,26 @@ cudaError_t device_alloc(void** out, size_t bytes) {
 // Lets entry points in other translation units record their error message.
 void set_last_error(const char* msg) { g_err = msg; }
 
-// A wide node's slot as the traversal reads it contains `box` (exact in
-// double: o is a float, s15 a power of two, the byte term 23 bits).
-static bool slot_contains(const WNode& w, int slot, const float box[6]) {
+// Whether a wide node's slots, as the traversal reads them, contain their boxes
+// (NULL: an empty slot) and are no looser than the packing makes them: planes
+// within four quanta (three and the roundings: two in the node's origin, one in
+// the byte), a quantum at most 1/124 of the node's extent (the next power of
+// two from 1/250), one ulp of its largest coordinate, or the least quantum.
+// Exact in double: o is a float, s15 a power of two, the byte term 23 bits.
+static bool slots_fit(const WNode& w, const float* const box[4]) {
   for (int k = 0; k < 3; k++) {
-    const double ql = (w.lo[k] >> (8 * slot)) & 255u, qh = (w.hi[k] >> (8 * slot)) & 255u;
-    const double o = w.o[k], s = w.s15[k];
-    if (!(o + (s + ql * (s / 32768.0)) <= (double)box[k]) || !((double)box[3 + k] <= o + (s + qh * (s / 32768.0))))
-      return false;
+    double og = INFINITY, hm = -INFINITY;
+    for (int s = 0; s < 4; s++)
+      if (box[s]) og = std::fmin(og, (double)box[s][k]), hm = std::fmax(hm, (double)box[s][3 + k]);
+    const double o = w.o[k], s15 = w.s15[k], q = s15 / 32768.0, big = std::fmax(std::fabs(og), std::fabs(hm));
+    const double ulp = big > 0.0 ? std::ldexp(1.0, std::ilogb(big) - 23) : 0.0;
+    if (!(q <= std::fmax((hm - og) / 124.0, std::fmax(ulp, std::ldexp(1.0, -63))))) return false;
+    for (int s = 0; s < 4; s++)
+      if (box[s]) {
+        const double lo = o + (s15 + ((w.lo[k] >> (8 * s)) & 255u) * q), hi = o + (s15 + ((w.hi[k] >> (8 * s)) & 255u) * q);
+        if (!(lo <= (double)box[s][k] && (double)box[s][k] - lo <= 4.0 * q)) return false;
+        if (!((double)box[s][3 + k] <= hi && hi - (double)box[s][3 + k] <= 4.0 * q)) return false;
+      }
   }
   return true;
 }
@@ -291,25 +303,20 @@ bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* 
     }
   }
   if (numbers && n > 1 && std::memcmp(boxes, root_box, 6 * sizeof(float)) != 0) return false;
-  // every slot of every wide node names the right node and contains its box (where the traversal looks at boxes)
+  // every slot of every wide node names the right node and fits its box (where the traversal looks at boxes)
   bool filtered = numbers;
   for (int c = 0; c < 6; c++) filtered = filtered && std::fabs(root_box[c]) <= kMaxFilterCoord;
-  auto code_of = [&](int x) { return x < ni ? x : ~(x - ni); };
-  for (int i = 0; i < ni; i++)
+  for (int i = 0; i < ni; i++) {
+    const float* box[4] = {};
     for (int s = 0; s < 4; s++) {
       const int c = nodes3[3 * i + 1 + (s >> 1)];
-      int x = c;
-      if (c >= ni) {
-        if (s & 1) {
-          if (wn[i].code[s] != kNoChild) return false;
-          continue;
-        }
-      } else {
-        x = nodes3[3 * c + 1 + (s & 1)];
-      }
-      if (wn[i].code[s] != code_of(x) || (filtered && !slot_contains(wn[i], s, boxes + 6 * (size_t)x)))
-        return false;
+      const bool used = c < ni || !(s & 1);  // (a leaf child takes its even slot)
+      const int x = c < ni ? nodes3[3 * c + 1 + (s & 1)] : c;
+      if (wn[i].code[s] != (!used ? kNoChild : (x < ni ? x : ~(x - ni)))) return false;
+      if (used) box[s] = boxes + 6 * (size_t)x;
     }
+    if (filtered && !slots_fit(wn[i], box)) return false;
+  }
   return true;
 }
 }  // namespace crt

@@ -102,7 +102,7 @@ cudaError_t device_alloc(void** out, size_t bytes);
 // from the parent words (relative to the tree, n >= 1 leaves), the boxes from
 // the leaves' triangles by exact unions.  false when the tree is inconsistent:
 // among the checks, the root box is the device's, and every slot of every wide
-// node names its node and contains that node's box.
+// node names its node and fits that node's box.
 bool export_tree(int n, const uint32_t* parent, const WNode* wn, const LeafTri* leaves, const float* root_box,
                  int* nodes3, float* boxes);
 
