@@ -791,18 +791,19 @@ static void refit(const MeshBufs& m, const BuildBufs& b, cudaStream_t st) {
 }
 
 // The cooperative sort's shape (items per thread) for n keys, -1 when it does
-// not take them: the fewest items that leave no more tiles than SMs, so that as
-// many SMs as possible rank keys.  (With 8 items whatever n, 19,220 keys were
-// three tiles and took 57 us; a 100,000-triangle build falls from 109 to 92 us,
-// 40,000 from 117 to 78, 19,220 from 84 to 61; at 1,003,520 7 items instead of
-// 8 and the shorter barrier make it 211.5 us from 216.5.)  The build takes it
-// from kCoopBuildMin keys on: below, three look-back passes launched as
-// programmatic dependents cost less than the cooperative launch (2000
-// triangles 43 against 54 us, 16,000 57.7 against 61.6, 19,220 58.1 against 60.9; 40,000
-// 74.8 against 73.9, 100,000 101.6 against 82.3).  The standalone sort,
-// which would also need a histogram pass, takes it from 1025 keys on (3000
-// 16-bit keys 55 against 64 us, 20,000 32-bit ones 73 against 78, 1,000,003
-// 131 against 137).
+// not take them: the fewest items of kCoopItems that leave no more tiles than
+// SMs, so that as many SMs as possible rank keys.  (3, 5 and 6 items are not
+// instantiated: 311,297 to 466,944 keys take 4, 622,593 to 933,888 take 7.
+// With 8 items whatever n, a build of 40,000 triangles takes 94.4 us instead of
+// 73.5, of 100,000 105.0 instead of 82.2, of 1,003,520 203.4 instead of 200.4.)
+// The build takes it from kCoopBuildMin keys on, where the curves meet: below,
+// three look-back passes launched as programmatic dependents cost less than the
+// cooperative launch (2000 triangles 42.0 against 49.6 us, 16,000 56.5 against
+// 59.7, 32,768 71.5 against 72.0, 40,000 74.2 against 73.5, 100,000 101.4
+// against 82.2, 1,003,520 201.4 against 200.4).  The standalone sort, which
+// would also need a histogram pass, takes it from 1025 keys on (3000 16-bit
+// keys 51 us with look-back passes, 43 with it; 20,000 32-bit ones 76 and 63;
+// 1,000,003 132 and 101).
 constexpr int kCoopBuildMin = 4 * kSortTileL, kCoopSortMin = kSortThreadsL + 1;
 using CoopSort = void (*)(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, int, int,
                           uint32_t*, unsigned*, int*);
@@ -1073,7 +1074,9 @@ cudaError_t launch_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t
   uint32_t* hist = w + 2 * (size_t)n;
   uint32_t* status = hist + passes * kRadix;
   unsigned* counters = status + (size_t)passes * tiles * kRadix;
-  // (one pass leaves room for half the rows that 1024-key tiles need)
+  // (sorts of one pass, key_bits <= 10, still take the look-back pass; the
+  // cooperative launch would be the faster one there too: 100,000 keys 50 us
+  // against 36, 1,000,003 59 against 48)
   const int shape = passes >= 2 ? coop_shape(n, kCoopSortMin, st) : -1;
   if (shape >= 0) {
     const cudaError_t e = cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), st);
